@@ -44,7 +44,7 @@ def listed():
         # first token of the headline request
         text("prompt 1616", "grouped", "prompt", 1, 1616, kv="scaled_fp8"),
         # a prompt step that batches several requests
-        text("prompts, 8 up to 1500", "grouped", "prompt", 8, 1500, even=False),
+        text("prompts 8 up to 1500", "grouped", "prompt", 8, 1500, even=False),
         # the last chunk of a long prompt, over the cached ones before it
         text("chunk 2048 after 14336", "grouped", "prompt", 1, 2048, history=14336, kv="scaled_fp8"),
         # the images of the headline request
