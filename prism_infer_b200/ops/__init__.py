@@ -62,11 +62,15 @@ def choose_splits(m: int, k: int, tokens: int) -> int:
         return 1
     tiles = (m + 127) // 128
     if tokens > 128:
-        tiles *= (tokens + 255) // 256  # upper bound of the kernel's own tile choice (128 or 256 tokens)
+        tiles *= (tokens + 255) // 256
     kb = (k + 63) // 64
     # one CTA per SM is resident (the operand ring fills shared memory), so more CTAs than
     # SMs means a second, mostly empty wave: stay at or below the SM count
     want = max(1, SM_COUNT // tiles)
+    if tokens > 128 and tiles >= 16:
+        # the SM pairs' kernel picks its tile width too: two slabs of a 4096-wide projection fill the pairs with 128 columns, and
+        # further slabs cost more in 32-bit partials than their shorter sums give
+        want = min(want, 2)
     return max(1, min(want, kb // 4 if kb >= 8 else 1, 16))
 
 

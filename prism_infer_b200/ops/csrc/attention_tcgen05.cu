@@ -100,7 +100,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   float* mx_s = reinterpret_cast<float*>(tmem_slot + 4);  // [2 buffers][2 halves][128 rows] maxima, then [2 halves][128 rows] sums
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // late query tiles see the most keys under a causal mask: schedule them first
   const int seq = blockIdx.z, head = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;
   const int kvh = head / (a.Hq / a.Hkv);
@@ -147,7 +147,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
 
   if (warp == 0) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       // ------------------------------ TMA producer ------------------------------
       constexpr bool TWO = HD_PAD > 64;
       mbar_expect_tx(q_full, TWO ? Q_BYTES : Q_BYTES / 2);
@@ -176,7 +176,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
       constexpr uint32_t IDESC_S = umma_idesc_bf16(FA_BM, FA_BN);
       constexpr uint32_t IDESC_O = umma_idesc_bf16(FA_BM, HD_PAD) | UMMA_B_MN_MAJOR;

@@ -207,6 +207,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int ta
   prism_report(PRISM_ERR_MBAR_TIMEOUT, tag);
   return false;
 }
+// One lane of a converged warp, chosen by the hardware.  The issuing roles branch on this and not on lane == 0: tcgen05 and TMA
+// instructions take their operands from uniform registers, and only behind elect.sync does the compiler know that a single lane
+// is active and move them there directly; behind lane == 0 each instruction is wrapped in a loop over the active lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok));
+  return ok != 0;
+}
+// Index of the warp in its block, in a form that the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

@@ -1,6 +1,6 @@
 // Weight-stationary-in-M GEMM family for sm_100a:  D[feature, token] = W[feature, :] . X[token, :]
 //
-// Every linear layer of the engine goes through this one kernel.  The weight matrix
+// Linear layers of up to 128 tokens go through this kernel (longer prompts: gemm_pair.cuh).  The weight matrix
 // (nn.Linear layout [out_features, in_features], i.e. K-major) is the tcgen05 A operand
 // with a fixed 128-row tile; the activations [tokens, in_features] (also K-major) are the
 // B operand with a token tile BN in {16, 32, 64, 128, 256}.  A decode step with a handful
@@ -33,6 +33,8 @@
 #include "common.cuh"
 
 PRISM_DEFINE_TU_STATUS(gemm)
+
+#include "gemm_pair.cuh"
 
 namespace {
 
@@ -109,7 +111,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   uint64_t* tmem_full = empty + stages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   // Rasterisation.  When the weight matrix does not fit the 126 MB L2, token tiles vary
   // fastest so the CTAs that share a weight tile run together and it leaves DRAM once;
@@ -151,7 +153,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   pdl_launch_dependents();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------ TMA producer ------------------------------
       const int pre = min(stages, num_kb);
       for (int i = 0; i < pre; ++i) {
@@ -165,35 +167,36 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         uint8_t* st = smem + (size_t)i * STAGE_BYTES;
         tma_load_2d(st + W_STAGE_BYTES, &tmX, &full[i], (kb_begin + i) * BK, n0);
       }
-      int issued = pre;
+      int s = 0;             // more k-blocks than stages: the next one reuses the first stage
+      uint32_t parity = 0;   // of its empty barrier
       bool ok = true;
-      for (int kb = pre; kb < num_kb && ok; ++kb) {
-        const int s = kb % stages;
-        const uint32_t round = kb / stages;
-        ok = mbar_wait(&empty[s], (round - 1) & 1, 1);
+      for (int kb = pre; kb < num_kb; ++kb) {
+        ok = mbar_wait(&empty[s], parity, 1);
         if (!ok) break;
         uint8_t* st = smem + (size_t)s * STAGE_BYTES;
         mbar_expect_tx(&full[s], STAGE_BYTES);
         tma_load_2d(st, &tmW, &full[s], (kb_begin + kb) * BK, w_row);
         if (DUAL) tma_load_2d(st + W_TILE_BYTES, &tmW, &full[s], (kb_begin + kb) * BK, a.w2_row_off + w_row);
         tma_load_2d(st + W_STAGE_BYTES, &tmX, &full[s], (kb_begin + kb) * BK, n0);
-        issued = kb + 1;
+        if (++s == stages) s = 0, parity ^= 1;
       }
       if (!ok) {
         // Unwinding after a timed-out wait: let copies already in flight land before the
-        // CTA's shared memory is released.
-        for (int kb = max(0, issued - stages); kb < issued; ++kb) {
-          (void)mbar_wait(&full[kb % stages], (kb / stages) & 1, 4);
+        // CTA's shared memory is released.  The stages before s are one round ahead of those from s on.
+        for (int j = 0; j < stages; ++j) {
+          if (--s < 0) s = stages - 1, parity ^= 1;
+          (void)mbar_wait(&full[s], parity ^ 1, 4);
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
       bool ok = true;
+      int s = 0;
+      uint32_t parity = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % stages;
-        ok = mbar_wait(&full[s], (kb / stages) & 1, 2);
+        ok = mbar_wait(&full[s], parity, 2);
         if (!ok) break;
         tc_fence_after();
         const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
@@ -209,6 +212,7 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           }
         }
         tc_commit(&empty[s]);
+        if (++s == stages) s = 0, parity ^= 1;
       }
       if (ok) tc_commit(tmem_full);
     }
@@ -386,12 +390,11 @@ gemm_wx_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
 
 
 // ------------------------------------------------------------------------------------
-// Persistent form for prefill-sized problems (no split-K, bf16 output, or fp32 with tokens on the lanes): one CTA per SM walks
-// a strided list of output tiles.  The TMA producer runs ahead across tile boundaries, the
-// MMA thread alternates between two TMEM accumulators when both fit (BN * (DUAL ? 2 : 1)
-// <= 256 columns), and the epilogue warps drain one accumulator while the next tile's MMAs
-// run, so tile set-up, pipeline fill and the store loop are off the tensor pipe's critical
-// path.
+// Persistent form on single SMs (no split-K, bf16 output): the experts of a prompt, the fused GEMM -> reduce-scatter, and prompts
+// whose rows are not 16-byte vectors; other prompts run gemm_pair.cuh.  One CTA per SM walks a strided list of output tiles.  The
+// TMA producer runs ahead across tile boundaries, the MMA thread alternates between two TMEM accumulators when both fit (BN *
+// (DUAL ? 2 : 1) <= 256 columns), and the epilogue warps drain one accumulator while the next tile's MMAs run, so tile set-up,
+// pipeline fill and the store loop are off the tensor pipe's critical path.
 // ------------------------------------------------------------------------------------
 struct PersistArgs {
   int dual_rm;  // row-major form only: the B tile is 128 gate rows followed by 128 up rows, epilogue = SwiGLU
@@ -400,7 +403,6 @@ struct PersistArgs {
   int tokens_fastest;
   int act;
   float glu_limit;   // bound of a bounded gated unit
-  int out_f32;  // row-major form without residual or scatter: out is float
   long long ldo, ldr;
   const __nv_bfloat16* bias;
   const __nv_bfloat16* residual;
@@ -416,17 +418,14 @@ struct PersistArgs {
   int* cta_counter;
   __nv_bfloat16* peer_out[8];
   unsigned long long* peer_flag[8];
-  PrismSections sec;  // row-major form only; row ends are multiples of 16 (a chunk lies in one section)
   const int4* groups;  // grouped form (row-major): token tile i is entry i of the table, m_tiles its capacity
   const int* n_groups;
   int group_rows;      // weight rows per expert
 };
 
-// ROWMAJOR: the A operand (128-row tiles, TMEM lanes) holds the tokens and B the weights, so an
-// epilogue thread owns one token row and 16 consecutive features per TMEM load: bias, residual
-// and output move as 16-byte vectors instead of sixteen strided 2-byte accesses (the strided
-// residual loads made the vision projections 6x slower than their main loop).  In that form
-// a.M counts tokens and a.T features.
+// ROWMAJOR: the A operand (128-row tiles, TMEM lanes) holds the tokens and B the weights, so an epilogue thread owns one token
+// row and stores 16 consecutive features per TMEM load as 16-byte vectors.  In that form a.M counts tokens and a.T features; it
+// serves the experts of a prompt (gated unit or plain) and the fused GEMM -> reduce-scatter (plain).
 template <int BN, bool DUAL, bool ROWMAJOR = false, bool GROUPED = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
@@ -448,7 +447,7 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
   uint64_t* acc_empty = acc_full + 2;    // [NBUF] epilogue -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
   int m_tiles = a.m_tiles;
   if (GROUPED) {
@@ -493,20 +492,19 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
   const int n0_ = (a.tokens_fastest ? (tile_) % a.n_tiles : (tile_) / m_tiles) * BN;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------ TMA producer ------------------------------
       pdl_wait();  // activations come from the previous kernel
-      long long it = 0;  // running k-block count across tiles
+      // Stage and parity are carried along: a 64-bit division by the number of stages for every k-block cost 800 cycles of the
+      // issuing threads, more than the 512 of the tile's MMAs.
+      int s = 0;
+      uint32_t parity = 1;  // of the empty barrier: a fresh one counts as free
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         PRISM_TILE_COORDS(tile, m0, n0)
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = (int)(it % stages);
-          const uint32_t round = (uint32_t)(it / stages);
-          if (round > 0) {
-            ok = mbar_wait(&empty[s], (round - 1) & 1, 1);
-            if (!ok) break;
-          }
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait(&empty[s], parity, 1);
+          if (!ok) break;
           uint8_t* st = smem + (size_t)s * STAGE_BYTES;
           mbar_expect_tx(&full[s], STAGE_BYTES);
           tma_load_2d(st, &tmW, &full[s], kb * BK, m0);
@@ -518,20 +516,23 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
           } else {
             tma_load_2d(st + W_STAGE_BYTES, &tmX, &full[s], kb * BK, w0 + n0);
           }
+          if (++s == stages) s = 0, parity ^= 1;
         }
       }
       if (!ok) {
         // unwinding after a timed-out wait: let copies already in flight land before the
         // CTA's shared memory is released
-        for (long long j = it - stages < 0 ? 0 : it - stages; j < it; ++j)
-          (void)mbar_wait(&full[j % stages], (uint32_t)(j / stages) & 1, 4);
+        for (int j = 0; j < stages; ++j) {
+          if (--s < 0) s = stages - 1, parity ^= 1;
+          (void)mbar_wait(&full[s], parity ^ 1, 4);
+        }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ------------------------------ MMA issuer ------------------------------
-      long long it = 0;
-      int local = 0;
+      int s = 0, local = 0;
+      uint32_t parity = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
         const int buf = local % NBUF;
@@ -542,9 +543,8 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
           tc_fence_after();
         }
         const uint32_t acc_addr = tmem_base + buf * ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = (int)(it % stages);
-          ok = mbar_wait(&full[s], (uint32_t)(it / stages) & 1, 2);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait(&full[s], parity, 2);
           if (!ok) break;
           tc_fence_after();
           const uint32_t st = smem_u32(smem + (size_t)s * STAGE_BYTES);
@@ -560,6 +560,7 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
             }
           }
           tc_commit(&empty[s]);
+          if (++s == stages) s = 0, parity ^= 1;
         }
         if (ok) tc_commit(&acc_full[buf]);
       }
@@ -616,59 +617,6 @@ gemm_wx_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
           float v[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-          int act = a.act;
-          if (a.sec.n > 0) {
-            float alpha;
-            prism_section_of(a.sec, f0, alpha, act);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] *= alpha;
-          }
-          if (a.bias != nullptr) {
-            const uint4 b0 = *reinterpret_cast<const uint4*>(a.bias + f0), b1 = *reinterpret_cast<const uint4*>(a.bias + f0 + 8);
-            const __nv_bfloat162* p0 = reinterpret_cast<const __nv_bfloat162*>(&b0);
-            const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&b1);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 x0 = __bfloat1622float2(p0[e]), x1 = __bfloat1622float2(p1[e]);
-              v[2 * e] += x0.x;
-              v[2 * e + 1] += x0.y;
-              v[8 + 2 * e] += x1.x;
-              v[8 + 2 * e + 1] += x1.y;
-            }
-          }
-          if (act == PRISM_ACT_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gelu_tanh(v[j]);
-          } else if (act == PRISM_ACT_GELU_ERF) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gelu_erf(v[j]);
-          } else if (act == PRISM_ACT_SIGMOID) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = sigmoid_fast(v[j]);
-          } else if (act == PRISM_ACT_DECAY) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = decay_of(v[j]);
-          }
-          if (a.residual != nullptr) {
-            const __nv_bfloat16* rs = a.residual + (size_t)m * a.ldr + f0;
-            const uint4 r0 = *reinterpret_cast<const uint4*>(rs), r1 = *reinterpret_cast<const uint4*>(rs + 8);
-            const __nv_bfloat162* p0 = reinterpret_cast<const __nv_bfloat162*>(&r0);
-            const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&r1);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 x0 = __bfloat1622float2(p0[e]), x1 = __bfloat1622float2(p1[e]);
-              v[2 * e] = bf16_round(v[2 * e]) + x0.x;
-              v[2 * e + 1] = bf16_round(v[2 * e + 1]) + x0.y;
-              v[8 + 2 * e] = bf16_round(v[8 + 2 * e]) + x1.x;
-              v[8 + 2 * e + 1] = bf16_round(v[8 + 2 * e + 1]) + x1.y;
-            }
-          }
-          if (a.out_f32) {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + (size_t)m * a.ldo + f0);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-            continue;
-          }
           uint4 o[2];
           __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(o);
 #pragma unroll
@@ -856,6 +804,16 @@ int g_persistent_min_tokens = 512;  // 0 disables the persistent form
 int g_persistent_rowmajor = 1;      // 1: tokens on the TMEM lanes for the non-dual persistent GEMM
 int g_sm_count = 0;
 
+int sm_count() {
+  if (g_sm_count == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      g_sm_count = 148;
+  }
+  return g_sm_count;
+}
+
+
 template <int BN, bool DUAL, bool ROWMAJOR = false, bool GROUPED = false>
 int launch_persistent(const CUtensorMap& tw, const CUtensorMap& tx, PersistArgs& a, cudaStream_t stream, bool pdl) {
   constexpr int STAGE_BYTES = W_TILE_BYTES * (DUAL ? 2 : 1) + BN * BK * 2;
@@ -870,14 +828,43 @@ int launch_persistent(const CUtensorMap& tw, const CUtensorMap& tx, PersistArgs&
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  if (g_sm_count == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      g_sm_count = 148;
-  }
   const int tiles = a.m_tiles * a.n_tiles;
-  const int grid = tiles < g_sm_count ? tiles : g_sm_count;
+  const int grid = tiles < sm_count() ? tiles : sm_count();
   return (int)prism_launch(gemm_wx_persistent_kernel<BN, DUAL, ROWMAJOR, GROUPED>, dim3(grid), dim3(GEMM_THREADS), smem, stream, pdl, tw, tx, a);
+}
+
+// Columns of a pair's tile.  A k-block of a tile takes 390 cycles (issue and barriers) or 2.7 per column, whichever is longer
+// (measured over 64 to 256 columns), and the launch as many rounds of tiles as the pairs need: 1616 x 4096 -> 4096 took 44 us with
+// 224 columns (two rounds of a few more columns than half of 256), 47 with 256, 56 with 128.
+int pair_columns(int m_tiles, int columns, bool dual) {
+  const int pairs = sm_count() / 2, step = dual ? 64 : 32;
+  int best = 64;
+  long long best_cost = 0;
+  for (int bn = 64; bn <= 256; bn += step) {
+    const long long rounds = ((long long)m_tiles * ((columns + bn - 1) / bn) + pairs - 1) / pairs;
+    const long long cost = rounds * ((bn < 144 ? 144 : bn) + 8);
+    if (best_cost == 0 || cost < best_cost) best = bn, best_cost = cost;
+  }
+  return best;
+}
+
+int launch_pair(const void* W, const void* X, int K, long long ldw, long long ldx, int w_rows, PairArgs& a, cudaStream_t stream, bool pdl) {
+  a.m_tiles = (a.T + 255) / 256;
+  a.bn = pair_columns(a.m_tiles * a.splits, a.N, a.dual != 0);
+  a.n_tiles = (a.N + a.bn - 1) / a.bn;
+  const int stage_bytes = W_TILE_BYTES + a.bn * 64;
+  a.stages = (SMEM_LIMIT - 1024 - 512) / stage_bytes;
+  if (a.stages > 12) a.stages = 12;
+  const size_t smem = (size_t)a.stages * stage_bytes + 1024 + (2 * a.stages + 4) * 8 + 64;
+  CUtensorMap tx, tw;
+  int rc = get_tensor_map(X, (unsigned long long)a.T, (unsigned long long)K, (unsigned long long)ldx, 128, &tx);
+  if (rc) return rc;
+  rc = get_tensor_map(W, (unsigned long long)w_rows, (unsigned long long)K, (unsigned long long)ldw, (unsigned)(a.bn / 2), &tw);
+  if (rc) return rc;
+  static const cudaError_t configured = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT);
+  if (configured != cudaSuccess) return (int)configured;
+  const int tiles = a.m_tiles * a.n_tiles * a.splits, pairs = sm_count() / 2;
+  return (int)prism_launch(gemm_pair_kernel, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(PAIR_THREADS), smem, stream, pdl, tx, tw, a);
 }
 
 }  // namespace
@@ -1002,12 +989,35 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
   if (rc) return rc;
   const int m_tiles = (M + BM - 1) / BM;
   const bool p = pdl != 0;
-  if (g_persistent_min_tokens > 0 && T >= g_persistent_min_tokens && splits == 1 && (!out_f32 || sections != nullptr) && push == nullptr &&
-      bn_override <= 0 && stages_override <= 0 &&
-      (sections == nullptr || (sections_rowmajor && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 &&
-                               ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0))) {
+  const bool plan_own = push == nullptr && bn_override <= 0 && stages_override <= 0 && g_persistent_min_tokens > 0;
+  const unsigned long long vec_addr = reinterpret_cast<unsigned long long>(out) | reinterpret_cast<unsigned long long>(bias) |
+                                      reinterpret_cast<unsigned long long>(residual);
+  // SM pairs, tokens on the TMEM lanes: from 129 tokens, where two CTAs have rows of their own, if the epilogue can move 16-byte
+  // vectors.  4096 -> 4096: 230 tokens 17 us (split-K form below 33), 1616 tokens 44 us (one-SM persistent form 64).
+  if (plan_own && T > 128 && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 && split_stride % 4 == 0 && (residual == nullptr || ldr % 8 == 0) &&
+      (vec_addr & 15ull) == 0 && (!dual || (bias == nullptr && residual == nullptr)) && (!out_f32 || sections != nullptr || (bias == nullptr && residual == nullptr && act == 0)) &&
+      (sections == nullptr || sections_rowmajor)) {
+    PairArgs g = {};
+    g.T = T;
+    g.N = dual ? 2 * M : M;
+    g.kb_total = a.kb_total;
+    g.splits = splits;
+    g.kb_per_split = a.kb_per_split;
+    g.split_stride = split_stride;
+    g.dual = dual;
+    g.up_row = w2_row_off;
+    g.act = act;
+    g.out_f32 = out_f32;
+    g.ldo = ldo;
+    g.ldr = ldr;
+    g.bias = a.bias;
+    g.residual = a.residual;
+    g.out = out;
+    g.sec = a.sec;
+    return launch_pair(W, X, K, ldw, ldx, w_rows_total, g, stream, p);
+  }
+  if (plan_own && T >= g_persistent_min_tokens && splits == 1 && !out_f32 && sections == nullptr) {
     PersistArgs pa;
-    pa.sec = a.sec;
     pa.groups = nullptr;
     pa.n_groups = nullptr;
     pa.group_rows = 0;
@@ -1018,7 +1028,6 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
     pa.m_tiles = m_tiles;
     pa.tokens_fastest = a.tokens_fastest;
     pa.act = act;
-    pa.out_f32 = out_f32;
     pa.ldo = ldo;
     pa.ldr = ldr;
     pa.bias = a.bias;
@@ -1035,46 +1044,7 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
       pa.peer_out[i] = nullptr;
       pa.peer_flag[i] = nullptr;
     }
-    const unsigned long long vec_addr = reinterpret_cast<unsigned long long>(out) | reinterpret_cast<unsigned long long>(bias) |
-                                        reinterpret_cast<unsigned long long>(residual);
     pa.dual_rm = 0;
-    if (dual && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 && (vec_addr & 15ull) == 0 && bias == nullptr &&
-        residual == nullptr) {
-      // gated unit with tokens on the TMEM lanes: one N = 256 MMA per step over [128 gate rows | 128 up rows]
-      CUtensorMap ta, tb;
-      rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, BM, &ta);
-      if (rc) return rc;
-      rc = get_tensor_map(W, (unsigned long long)w_rows_total, (unsigned long long)K, (unsigned long long)ldw, 128, &tb);
-      if (rc) return rc;
-      pa.dual_rm = 1;
-      pa.M = T;
-      pa.T = 2 * M;                       // accumulator columns per full sweep: gate + up
-      pa.m_tiles = (T + BM - 1) / BM;
-      pa.n_tiles = (M + 127) / 128;       // 128 features (256 accumulator columns) per tile
-      pa.tokens_fastest = a.tokens_fastest ? 0 : 1;
-      return launch_persistent<256, false, true>(ta, tb, pa, stream, p);
-    }
-    if (!dual && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 && (residual == nullptr || ldr % 8 == 0) &&
-        (vec_addr & 15ull) == 0) {
-      // tokens on the TMEM lanes: vectorised bias / residual / output rows
-      pa.M = T;
-      pa.T = M;
-      pa.m_tiles = (T + BM - 1) / BM;
-      pa.tokens_fastest = a.tokens_fastest ? 0 : 1;  // the A-row tile index is the token tile here
-      // Always 256 weight rows per tile: 128-row tiles balance better over the SMs when there
-      // are few tiles, but they double the operand bytes per FLOP and measured 20-45% slower
-      // (1616 x 4096 -> 6144: 0.141 vs 0.097 ms).
-      const int n256 = (M + 255) / 256;
-      const bool narrow = false;
-      CUtensorMap ta, tb;
-      rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, BM, &ta);
-      if (rc) return rc;
-      rc = get_tensor_map(W, (unsigned long long)w_rows_total, (unsigned long long)K, (unsigned long long)ldw, narrow ? 128 : 256, &tb);
-      if (rc) return rc;
-      pa.n_tiles = n256;
-      return narrow ? launch_persistent<128, false, true>(ta, tb, pa, stream, p)
-                    : launch_persistent<256, false, true>(ta, tb, pa, stream, p);
-    }
     // dual: two accumulators per tile, so 128 tokens per tile keep two tiles in TMEM
     const int pbn = dual ? 128 : 256;
     pa.n_tiles = (T + pbn - 1) / pbn;
@@ -1177,7 +1147,6 @@ PRISM_API int prism_gemm_grouped(const void* W, const void* X, void* out, int M,
   if (act < 0 || act > PRISM_GLU_BOUNDED || ldo % 8 || (reinterpret_cast<uintptr_t>(out) & 15)) return -2;
   const bool dual = act != 0;
   PersistArgs pa = {};
-  pa.sec.n = 0;
   pa.dual_rm = dual ? 1 : 0;
   pa.M = N;
   pa.T = dual ? 2 * M : M;
@@ -1275,7 +1244,6 @@ PRISM_API int prism_gemm_wx_scatter(const void* W, const void* X, int M, int T, 
   rc = get_tensor_map(W, (unsigned long long)M, (unsigned long long)K, (unsigned long long)ldw, 256, &tb);
   if (rc) return rc;
   PersistArgs pa;
-  pa.sec.n = 0;
   pa.dual_rm = 0;
   pa.M = T;
   pa.T = M;
@@ -1285,7 +1253,6 @@ PRISM_API int prism_gemm_wx_scatter(const void* W, const void* X, int M, int T, 
   pa.n_tiles = (M + 255) / 256;
   pa.tokens_fastest = 0;
   pa.act = 0;
-  pa.out_f32 = 0;
   pa.ldo = M;
   pa.ldr = 0;
   pa.bias = nullptr;

@@ -773,7 +773,7 @@ window_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_empty + 4);
   float* xch = reinterpret_cast<float*>(tmem_slot + 4);              // [2][128] row sums, then [2][128] sums of squares
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int seq = blockIdx.z, qt = gridDim.x - 1 - blockIdx.x;       // late tiles first
   const int share = a.H / a.G;
   const bool tiles2 = a.maps == 1 && !p.pair_heads;                  // the streams are two query tiles
@@ -822,7 +822,7 @@ window_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   };
 
   if (warp == 0) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       // ------------------------------ TMA producer ------------------------------
       const bool two_q = !tiles2 || row_1 < q_len;
       mbar_expect_tx(q_full, (two_q ? 2 : 1) * q_bytes);
@@ -856,7 +856,7 @@ window_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int t = max(0, issued - p.stages); t < issued; ++t) (void)mbar_wait(&kv_full[t % p.stages], (t / p.stages) & 1, 42);
     }
   } else if (warp == 1 || warp == 10) {
-    if (lane == 0 && live) {
+    if (live && elect_one()) {
       // ------------------------------ MMA issuer of one stream ------------------------------
       const int s = warp == 1 ? 0 : 1;
       const uint32_t idesc_s = umma_idesc_bf16(PT, PKT);

@@ -527,3 +527,35 @@ def test_fp8_candidate_lm_head_finds_the_exact_argmax(cuda_device, B, V, H):
             assert int(got[b]) == int(want[b]) + 11, (b, int(got[b]), int(want[b]))
         else:
             assert float(logits[b, int(got[b]) - 11]) >= float(top2[b, 1]) - 1e-3
+
+
+@pytest.mark.parametrize("T,M,K", [(129, 16, 8), (130, 4096, 64), (256, 272, 1160), (257, 1152, 4304), (511, 4304, 1152), (1616, 3456, 448),
+                                   (2305, 528, 136)])
+@pytest.mark.parametrize("form", ["bias gelu residual", "gated", "slabs", "sections"])
+def test_gemm_on_sm_pairs(cuda_device, T, M, K, form):
+    """Prompt-sized products: ragged token, feature and depth tiles; every epilogue.  bf16 results: one or two roundings of 2^-9.  32-bit
+    results: K / 16 chained additions (the slabs' sums and the epilogue add a few), each off by 2^-23 of a running sum that stays below 4
+    (four standard deviations), times the largest alpha."""
+    x, w = rand_bf16(T, K, seed=71), rand_bf16(2 * M if form == "gated" else M, K, scale=K ** -0.5, seed=72)
+    y = x.double() @ w.double().t()
+    if form == "gated":
+        got = ops.gate_up_glu(x.cuda(), w.cuda(), "silu")
+        want = torch.nn.functional.silu(y[:, :M]) * y[:, M:]
+    elif form == "slabs":
+        got = ops.linear_partial(x.cuda(), w.cuda(), 3).sum(0)
+        want = y
+    elif form == "sections":
+        from prism_infer_b200.ops import latent as lat
+
+        cut = M // 2 // 16 * 16
+        sections = lat.Sections([(cut, 0.5, "sigmoid"), (M - cut, 2.0, None)] if cut else [(M, 2.0, None)])
+        got = lat.linear_sections(x.cuda(), w.cuda(), sections, out_f32=True)
+        want = torch.cat([torch.sigmoid(0.5 * y[:, :cut]), 2.0 * y[:, cut:]], 1)
+    else:
+        b, r = rand_bf16(M, seed=73), rand_bf16(T, M, seed=74)
+        buf = r.clone().cuda()
+        got = ops.linear(x.cuda(), w.cuda(), bias=b.cuda(), act="gelu", residual=buf, out=buf)   # in place
+        want = torch.nn.functional.gelu(y + b.double()) + r.double()
+    tol = 2.0 * 4.0 * (K / 16 + 16) * 2.0 ** -23 if got.dtype == torch.float32 else 1.2e-2
+    err = (got.double().cpu() - want).abs() / (1.0 + want.abs())
+    assert err.max() < tol, (form, err.max())
