@@ -195,81 +195,117 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(const AddNormArgs a) 
   }
 }
 
+// The form of add+RMSNorm for rows of 16-byte vectors (hidden size a multiple of 8, at most 8192), bf16 delta rows or fp32 slabs.
+// One CTA per row, NV vectors per thread.  Every load of the row is issued before its first store: residual_out may be residual_in,
+// so a load that follows a store in the program also follows it in time, and a loop that reads, adds and writes one vector after the
+// other waits for memory once per vector (1616 x 4096: 39 -> 12 us, 5100 x 4096: 165 -> 55 us; 128 rows of 4 slabs: 9 -> 4 us).
+// The norm weights come from no kernel and are read before the wait.  Same rounding points as add_rmsnorm_kernel.
 // ---------------------------------------------------------------------------------
-// Prefill form of add+RMSNorm (bf16 delta rows, hidden size at most 8192): one warp per row,
-// the pre-norm row lives in registers as 16-byte vectors, no shared memory or block barrier.
-// Same rounding points as add_rmsnorm_kernel.
-// ---------------------------------------------------------------------------------
-constexpr int RN_VEC = 32;  // vectors of 8 bf16 per lane (8192 / 32 / 8)
-template <int NV>
-__global__ void __launch_bounds__(256) add_rmsnorm_rows_kernel(const AddNormArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  pdl_launch_dependents();
-  pdl_wait();
-  if (t >= a.T) return;
-  const int H = a.H, nvec = H >> 3;
+constexpr int RN_MAX = 8192;
+template <int NV, bool SLABS>
+__global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNormArgs a) {
+  __shared__ float red[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int t = blockIdx.x, H = a.H, nvec = H >> 3;
   const size_t base = (size_t)t * H;
+  pdl_launch_dependents();
+  uint4 w[NV], r[NV], e[NV], v[NV];
+  if (a.out != nullptr) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = threadIdx.x + blockDim.x * k;
+      if (i < nvec) w[k] = reinterpret_cast<const uint4*>(a.weight)[i];
+    }
+  }
+  pdl_wait();
   const int ex = a.extra != nullptr ? a.extra_index[t] : -1;
-  uint4 v[NV];
+  float4 lo[NV], hi[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + blockDim.x * k;
+    if (i < nvec) {
+      if (a.residual_in != nullptr) r[k] = reinterpret_cast<const uint4*>(a.residual_in + base)[i];
+      if (ex >= 0) e[k] = reinterpret_cast<const uint4*>(a.extra + (size_t)ex * H)[i];
+      if (!SLABS) v[k] = reinterpret_cast<const uint4*>(a.x_in + base)[i];
+    }
+  }
+  if (SLABS) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) lo[k] = hi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int p = 0; p < a.P; ++p) {
+      const float4* src = reinterpret_cast<const float4*>(a.partials + (size_t)p * a.slab_stride + base);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + blockDim.x * k;
+        if (i < nvec) {
+          const float4 x = __ldcg(src + 2 * i), y = __ldcg(src + 2 * i + 1);
+          lo[k].x += x.x, lo[k].y += x.y, lo[k].z += x.z, lo[k].w += x.w;
+          hi[k].x += y.x, hi[k].y += y.y, hi[k].z += y.z, hi[k].w += y.w;
+        }
+      }
+    }
+  }
   float ss = 0.0f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = lane + 32 * k;
+    const int i = threadIdx.x + blockDim.x * k;
     if (i < nvec) {
-      uint4 x = reinterpret_cast<const uint4*>(a.x_in + base)[i];
-      __nv_bfloat162* xp = reinterpret_cast<__nv_bfloat162*>(&x);
-      float2 d[4];
+      __nv_bfloat162* vp = reinterpret_cast<__nv_bfloat162*>(&v[k]);
+      if (SLABS) {
+        vp[0] = __floats2bfloat162_rn(lo[k].x, lo[k].y);
+        vp[1] = __floats2bfloat162_rn(lo[k].z, lo[k].w);
+        vp[2] = __floats2bfloat162_rn(hi[k].x, hi[k].y);
+        vp[3] = __floats2bfloat162_rn(hi[k].z, hi[k].w);
+      }
+      const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&r[k]);
+      const __nv_bfloat162* ep = reinterpret_cast<const __nv_bfloat162*>(&e[k]);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) d[e] = __bfloat1622float2(xp[e]);
-      if (a.residual_in != nullptr) {
-        const uint4 r = reinterpret_cast<const uint4*>(a.residual_in + base)[i];
-        const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&r);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(rp[e]);
-          d[e].x = bf16_round(f.x + d[e].x);
-          d[e].y = bf16_round(f.y + d[e].y);
+      for (int j = 0; j < 4; ++j) {
+        float2 d = __bfloat1622float2(vp[j]);
+        if (a.residual_in != nullptr) {
+          const float2 f = __bfloat1622float2(rp[j]);
+          d.x = bf16_round(f.x + d.x);
+          d.y = bf16_round(f.y + d.y);
         }
-      }
-      if (ex >= 0) {
-        const uint4 r = reinterpret_cast<const uint4*>(a.extra + (size_t)ex * H)[i];
-        const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&r);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(rp[e]);
-          d[e].x = bf16_round(d[e].x + f.x);
-          d[e].y = bf16_round(d[e].y + f.y);
+        if (ex >= 0) {
+          const float2 f = __bfloat1622float2(ep[j]);
+          d.x = bf16_round(d.x + f.x);
+          d.y = bf16_round(d.y + f.y);
         }
+        ss += d.x * d.x + d.y * d.y;
+        vp[j] = __floats2bfloat162_rn(d.x, d.y);  // exact: the sums are already bf16 values
       }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        ss += d[e].x * d[e].x + d[e].y * d[e].y;
-        xp[e] = __floats2bfloat162_rn(d[e].x, d[e].y);  // exact: the sums are already bf16 values
-      }
-      v[k] = x;
-      if (a.residual_out != nullptr) reinterpret_cast<uint4*>(a.residual_out + base)[i] = x;
+      if (a.residual_out != nullptr) reinterpret_cast<uint4*>(a.residual_out + base)[i] = v[k];
     }
   }
-  const float rstd = rsqrtf(warp_sum(ss) / (float)H + a.eps);
   if (a.out == nullptr) return;
+  ss = warp_sum(ss);
+  if (lane == 0) red[warp] = ss;
+  __syncthreads();
+  const float rstd = rsqrtf(warp_sum(lane < warps ? red[lane] : 0.0f) / (float)H + a.eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = lane + 32 * k;
+    const int i = threadIdx.x + blockDim.x * k;
     if (i < nvec) {
-      const uint4 w = reinterpret_cast<const uint4*>(a.weight)[i];
-      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&w);
+      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&w[k]);
       const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&v[k]);
       uint4 o;
       __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = __bfloat1622float2(xp[e]), wf = __bfloat1622float2(wp[e]);
-        op[e] = __floats2bfloat162_rn(bf16_round(f.x * rstd) * wf.x, bf16_round(f.y * rstd) * wf.y);
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(xp[j]), wf = __bfloat1622float2(wp[j]);
+        op[j] = __floats2bfloat162_rn(bf16_round(f.x * rstd) * wf.x, bf16_round(f.y * rstd) * wf.y);
       }
       reinterpret_cast<uint4*>(a.out + base)[i] = o;
     }
   }
+}
+template <int NV>
+static int launch_add_rmsnorm_rows(const AddNormArgs& a, cudaStream_t stream, bool pdl) {
+  const int threads = ((a.H / 8 + NV - 1) / NV + 31) / 32 * 32;
+  return (int)(a.P > 0 ? prism_launch(add_rmsnorm_rows_kernel<NV, true>, dim3(a.T), dim3(threads), 0, stream, pdl, a)
+                       : prism_launch(add_rmsnorm_rows_kernel<NV, false>, dim3(a.T), dim3(threads), 0, stream, pdl, a));
 }
 
 // ---------------------------------------------------------------------------------
@@ -883,33 +919,59 @@ __global__ void __launch_bounds__(256) pos_embed_add_kernel(bf16* x, const bf16*
 
 // Vision 2-D rotary on q and k inside the packed [N][3][heads][hd] projection, in place.
 // angle[n][i] for i < hd/2: first hd/4 slots use the row coordinate, next hd/4 the column.
-__global__ void __launch_bounds__(256) vit_rope_kernel(bf16* qkv, const int* coords, const float* inv_freq, int N,
-                                                       int heads, int hd) {
-  // The angle depends on (patch, i) only: 36 sin/cos pairs per patch are computed once into
-  // shared memory, then every (q|k, head) row is rotated with 4-byte accesses.
+// The angle depends on (patch, i) only: its sines and cosines are computed once into shared memory, then every (q|k, head) row is
+// rotated.  V elements per access (8 bytes where half a head is a multiple of 4); both accesses of a thread are loaded before the
+// first is stored, since the rotation is in place (6272 patches x 16 heads of 72: 20 -> 16 us).
+template <int V>
+struct alignas(2 * V) BfVec {
+  __nv_bfloat162 p[V / 2];
+};
+template <int V>
+__global__ void __launch_bounds__(256) vit_rope_kernel(bf16* qkv, const int* coords, const float* inv_freq, int heads, int hd) {
   __shared__ float sn_s[128], cs_s[128];
   const int n = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
-  const int half = hd / 2, quarter = hd / 4;
-  if ((int)threadIdx.x < half) {
-    const int i = threadIdx.x;
-    const float pos = (float)coords[2 * n + (i < quarter ? 0 : 1)];
-    sincosf(pos * inv_freq[i % quarter], &sn_s[i], &cs_s[i]);
-  }
-  __syncthreads();
-  const int pairs = half / 2;  // two adjacent i per thread and step
-  const int work = 2 * heads * pairs;
-  for (int w = threadIdx.x; w < work; w += blockDim.x) {
-    const int i = (w % pairs) * 2;
-    const int h = (w / pairs) % heads;
-    const int which = w / (pairs * heads);  // 0 = q, 1 = k
-    bf16* p = qkv + ((size_t)n * 3 + which) * heads * hd + (size_t)h * hd;
-    const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + i));
-    const float2 x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + i + half));
-    const float c0 = cs_s[i], c1 = cs_s[i + 1], s0 = sn_s[i], s1 = sn_s[i + 1];
-    *reinterpret_cast<__nv_bfloat162*>(p + i) = __floats2bfloat162_rn(x0.x * c0 - x1.x * s0, x0.y * c1 - x1.y * s1);
-    *reinterpret_cast<__nv_bfloat162*>(p + i + half) = __floats2bfloat162_rn(x1.x * c0 + x0.x * s0, x1.y * c1 + x0.y * s1);
+  const int half = hd / 2, quarter = hd / 4, vecs = half / V, work = 2 * heads * vecs;
+  bf16* const row = qkv + (size_t)n * 3 * heads * hd;   // the 2 * heads rows of q and k follow one another
+  for (int w0 = threadIdx.x; w0 < work || w0 < (int)blockDim.x; w0 += 2 * blockDim.x) {
+    BfVec<V> x0[2], x1[2];
+    bf16* p[2];
+    int at[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int w = w0 + j * blockDim.x;
+      if (w < work) {
+        const int h = w / vecs;
+        at[j] = (w - h * vecs) * V;
+        p[j] = row + (size_t)h * hd + at[j];
+        x0[j] = *reinterpret_cast<const BfVec<V>*>(p[j]);
+        x1[j] = *reinterpret_cast<const BfVec<V>*>(p[j] + half);
+      }
+    }
+    if (w0 == (int)threadIdx.x) {
+      if ((int)threadIdx.x < half) {
+        const int i = threadIdx.x;
+        const float pos = (float)coords[2 * n + (i < quarter ? 0 : 1)];
+        sincosf(pos * inv_freq[i % quarter], &sn_s[i], &cs_s[i]);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (w0 + j * (int)blockDim.x < work) {
+        BfVec<V> y0, y1;
+#pragma unroll
+        for (int e = 0; e < V / 2; ++e) {
+          const float2 u = __bfloat1622float2(x0[j].p[e]), v = __bfloat1622float2(x1[j].p[e]);
+          const float c0 = cs_s[at[j] + 2 * e], c1 = cs_s[at[j] + 2 * e + 1], s0 = sn_s[at[j] + 2 * e], s1 = sn_s[at[j] + 2 * e + 1];
+          y0.p[e] = __floats2bfloat162_rn(u.x * c0 - v.x * s0, u.y * c1 - v.y * s1);
+          y1.p[e] = __floats2bfloat162_rn(v.x * c0 + u.x * s0, v.y * c1 + u.y * s1);
+        }
+        *reinterpret_cast<BfVec<V>*>(p[j]) = y0;
+        *reinterpret_cast<BfVec<V>*>(p[j] + half) = y1;
+      }
+    }
   }
 }
 
@@ -952,11 +1014,11 @@ static int add_rmsnorm_impl(const void* partials, long long slab_stride, int P, 
     const unsigned long long addr = reinterpret_cast<unsigned long long>(x_in) | reinterpret_cast<unsigned long long>(residual_in) |
                                     reinterpret_cast<unsigned long long>(residual_out) | reinterpret_cast<unsigned long long>(extra) |
                                     reinterpret_cast<unsigned long long>(weight) | reinterpret_cast<unsigned long long>(out);
-    if (T >= 64 && P == 0 && x_in != nullptr && n_wait == 0 && H % 8 == 0 && H <= 8192 && (addr & 15ull) == 0) {
-      dim3 grid((T + 7) / 8), block(256);
-      if (H <= 2048) return (int)prism_launch(add_rmsnorm_rows_kernel<8>, grid, block, 0, STREAM(stream), pdl != 0, a);
-      if (H <= 4096) return (int)prism_launch(add_rmsnorm_rows_kernel<16>, grid, block, 0, STREAM(stream), pdl != 0, a);
-      return (int)prism_launch(add_rmsnorm_rows_kernel<RN_VEC>, grid, block, 0, STREAM(stream), pdl != 0, a);
+    if (n_wait == 0 && !packed && H % 8 == 0 && H <= RN_MAX && (addr & 15ull) == 0 &&
+        (P > 0 ? (slab_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(partials) & 15) == 0) : x_in != nullptr)) {
+      // up to one row per SM: a vector per thread, the shortest chain; more: few enough threads that several rows share an SM
+      if (T <= 148) return launch_add_rmsnorm_rows<1>(a, STREAM(stream), pdl != 0);
+      return launch_add_rmsnorm_rows<4>(a, STREAM(stream), pdl != 0);
     }
   }
   // few rows: one wide CTA per row so every element has its own thread; many rows: 256 threads
@@ -1153,6 +1215,14 @@ PRISM_API int prism_vit_rope(void* qkv, const void* coords, const void* inv_freq
                              int pdl) {
   if (N <= 0) return 0;
   if (hd % 4 || hd > 256) return -1;
-  return (int)prism_launch(vit_rope_kernel, dim3(N), dim3(256), 0, STREAM(stream), pdl != 0, (bf16*)qkv,
-                           (const int*)coords, (const float*)inv_freq, N, heads, hd);
+  const bool wide = hd % 8 == 0 && (reinterpret_cast<uintptr_t>(qkv) & 7) == 0;
+  const int work = 2 * heads * (hd / 2) / (wide ? 4 : 2);
+  // two accesses per thread where a block of 256 can take them, and at least a thread per angle
+  int threads = ((work + 1) / 2 + 31) / 32 * 32;
+  threads = threads > 256 ? 256 : threads;
+  if (threads < hd / 2) threads = (hd / 2 + 31) / 32 * 32;
+  return wide ? (int)prism_launch(vit_rope_kernel<4>, dim3(N), dim3(threads), 0, STREAM(stream), pdl != 0, (bf16*)qkv, (const int*)coords,
+                                  (const float*)inv_freq, heads, hd)
+              : (int)prism_launch(vit_rope_kernel<2>, dim3(N), dim3(threads), 0, STREAM(stream), pdl != 0, (bf16*)qkv, (const int*)coords,
+                                  (const float*)inv_freq, heads, hd);
 }
