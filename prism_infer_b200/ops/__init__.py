@@ -581,8 +581,13 @@ def embed(ids: torch.Tensor, table: torch.Tensor, *, visual: Optional[torch.Tens
 
 # --------------------------------------------------------------------------- attention
 def decode_splits(batch: int, num_kv_heads: int) -> int:
-    want = max(1, (2 * SM_COUNT) // max(1, batch * num_kv_heads))
-    return int(min(32, want))
+    """Blocks that share the cached tokens of one (sequence, KV head): a power of two, whose blocks form a cluster and merge in
+    shared memory, at most 16 (the largest cluster) and at most 256 blocks in all (two and three of them fit an SM, and a call of more
+    than one round is slower: 8 sequences of up to 3000 tokens, 8 KV heads: 20 us with 2, 18 with 4, 22 with 8, 43 with 16)."""
+    n = 1
+    while n < 16 and 2 * n * batch * num_kv_heads <= 256:
+        n *= 2
+    return n
 
 
 _DECODE_COUNTERS: dict = {}

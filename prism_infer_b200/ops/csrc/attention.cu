@@ -46,6 +46,7 @@ struct DecodeArgs {
   int Hq, Hkv, page, max_blocks, nsplit;
   int num_blocks;           // pages in the cache; <= 0: unknown, only holes (< 0) are skipped
   float scale;
+  int clustered;            // the splits of a (sequence, KV head) are the blocks of one cluster and merge in shared memory
 };
 
 // KV8 = true: fp8 payload (16 elements per lane), false: bf16 payload (8 elements per lane)
@@ -584,195 +585,270 @@ __global__ void __launch_bounds__(BM * 2, MODE == 2 ? (BM == 128 ? 1 : 2) : (BM 
 }
 
 // =====================================================================================
-// Decode on the tensor cores (mma.sync m16n8k16): the G query heads of a KV head are rows of
-// one 16-row A tile, a 64-token K/V tile is dequantised to bf16 in shared memory once and
-// each warp scores and accumulates 16 of its tokens.  Used for larger batches, where the
-// SIMT kernel above is instruction-bound (one FMA per head and byte); same split-KV
-// partial format and in-kernel merge.
+// Decode on the tensor cores (mma.sync m16n8k16), at most 8 query heads per KV head, pages of whole 16-token steps.  Same split-KV
+// partial format and in-kernel merge as the kernel above where the splits are not a cluster; the splits of a cluster read each other's
+// partial sums from shared memory instead (write, fence, count and read back through memory took 4 us of a 13 us call).
+//
+// A decode step reads every cached byte once, so the kernel has to keep bytes in flight and spend few instructions on them.  Each
+// warp walks 16-token steps of its own: one lane asks TMA for the step's 16 K rows and 16 V rows (128-byte swizzle) a ring ahead,
+// ldmatrix reads them without bank conflicts, and no block barrier or per-lane address is left in the loop.
+//   * tokens are the M rows and the heads the 8 N columns: S = K Q^T, O^T = V^T P^T.  Nothing is padded but the heads.
+//   * P changes from rows of tokens to rows of heads with one movmatrix per 8 tokens.
+//   * 8-bit rows are read as pairs: the depth order of S and the row order of O^T are permuted to fit, and Q and the output follow.
+//     The scales multiply the scores and the probabilities, so K and V enter the products exactly.
+// Scores refer to a maximum that is raised only when a step exceeds it by more than 2^8; sums and accumulators are 32-bit.
+// The tile form before it (64 tokens dequantised in shared memory by the block, 240 registers, 8 warps per SM) took 1.8 us per tile
+// and SM whatever the format.  One sequence of 1650 tokens, 8 KV heads: 13.8 -> 8.8 us (8-bit); 32 of 512 to 2048: 62 -> 33 us (8-bit,
+// 84 MB; the longest sequence's chain of steps), 64 -> 33 us (bf16, 168 MB, 5.0 TB/s); 128 of 256 to 1024: 100 -> 57 us (bf16, 335 MB,
+// 5.8 TB/s), 94 -> 47 us (8-bit).  Copying fragments by lane (cp.async or loads into registers) measured 62 and 55 us for the second.
 // =====================================================================================
-template <int D, int G, bool KV8>
-__global__ void __launch_bounds__(128) paged_decode_mma_kernel(const DecodeArgs a) {
-  constexpr int BN = 64, NWARP = 4;
-  constexpr int LDS = D + 8;
-  constexpr int CHUNKS = D / 8;
-  extern __shared__ __align__(16) uint8_t dsm[];
-  bf16* Qs = reinterpret_cast<bf16*>(dsm);
-  bf16* Ks = Qs + 16 * LDS;
-  bf16* Vs = Ks + BN * LDS;
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t fp8x2_to_bf16x2(uint32_t v) {  // exact: E4M3 has three mantissa bits
+  const float2 f = fp8x2_to_float2((unsigned short)v);
+  return pack_bf16(f.x, f.y);
+}
+// Untiled copy; both addresses and the size are multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(src),
+               "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+template <int D, bool KV8>
+struct DecodeShape {
+  static constexpr int ATOMS = D * (KV8 ? 1 : 2) > 128 ? 2 : 1;  // 128-byte columns of a row
+  static constexpr int ROWS_BYTES = ATOMS * 2048;                // 16 rows of K, or of V
+  static constexpr int STEP_BYTES = 2 * ROWS_BYTES;
+  static constexpr int STAGES = ATOMS == 2 ? 3 : 4;              // two and three blocks of four warps per SM
+  static constexpr int RING = 4 * STAGES * STEP_BYTES;
+  static constexpr int SCALES = KV8 ? 4 * STAGES * 128 : 0;      // 16 scales of K, 16 of V
+  static constexpr int MERGE = 5 * 8 * D * 4;                    // the warps' sums and the block's, where the ring was
+  static_assert(MERGE <= RING, "the merge reuses the ring");
+  static constexpr int SMEM_BYTES = RING + SCALES + 1024;
+};
+
+template <int D, bool KV8>
+__global__ void __launch_bounds__(128, DecodeShape<D, KV8>::ATOMS == 2 ? 2 : 3)
+paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeArgs a) {
+  using Shape = DecodeShape<D, KV8>;
+  constexpr int NWARP = 4, STEP = 16, SPAN = NWARP * STEP, STAGES = Shape::STAGES, ATOMS = Shape::ATOMS;
+  constexpr int KT = D / 16;                 // depth steps of S, row tiles of O^T
+  extern __shared__ uint8_t dsm_raw[];
+  uint8_t* const dsm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ float s_m[NWARP][8], s_l[NWARP][8];
+  __shared__ uint64_t bars[NWARP][STAGES];
   const int b = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3;
+  const int G = a.Hq / a.Hkv;
+  uint8_t* const ring = dsm + warp * STAGES * Shape::STEP_BYTES;
+  float* const scale_ring = reinterpret_cast<float*>(dsm + Shape::RING) + warp * STAGES * 32;
+  if (lane == 0) {
+    for (int i = 0; i < STAGES; ++i) mbar_init(&bars[warp][i], 1);
+    fence_barrier_init();
+  }
   pdl_launch_dependents();
+  __syncwarp();
   pdl_wait();
   const int ctx = clamp_context(a.context_lens[b], a.max_blocks, a.page);
-  const int per_split = ((ctx + a.nsplit - 1) / a.nsplit + BN - 1) / BN * BN;
-  const int j_begin = split * per_split;
-  const int j_end = min(ctx, j_begin + per_split);
+  // Every split but the last takes the same number of whole spans.  With the in-kernel merge, splits without tokens leave at once:
+  // they neither write partials nor count as arrivals, so a short context does not pay for the splits of a long one.
+  const int spans = (ctx + SPAN - 1) / SPAN, per_split = (spans + a.nsplit - 1) / a.nsplit * SPAN;
+  const int used = a.counters == nullptr && !a.clustered ? a.nsplit : max(1, (ctx + per_split - 1) / max(1, per_split));
+  if (split >= used && !a.clustered) return;
+  const int j_begin = split * per_split + warp * STEP, j_end = min(ctx, (split + 1) * per_split);
   const int* bt = a.block_tables + (size_t)b * a.max_blocks;
 
-  for (int i = tid; i < 16 * CHUNKS; i += 128) {
-    const int r = i / CHUNKS, c = i % CHUNKS;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r < G) v = *reinterpret_cast<const uint4*>(a.q + ((size_t)b * a.Hq + (size_t)kvh * G + r) * D + c * 8);
-    *reinterpret_cast<uint4*>(Qs + r * LDS + c * 8) = v;
-  }
-  __syncthreads();
-  uint32_t qf[D / 16][4];
-  {
-    const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
-    const int c = 8 * (lane >> 4);
-#pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) ldsm_x4(qf[kk], smem_u32(Qs + r * LDS + kk * 16 + c));
-  }
-  float o[D / 8][4];
-#pragma unroll
-  for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-  float m_run = -INFINITY, l_run = 0.0f;  // row g (rows >= G are padding)
-  const float sl2 = a.scale * 1.4426950408889634f;
-
-  // Software pipeline: the global loads of tile i+1 are in flight (in registers) while
-  // tile i is scored; 16-byte loads, CPR chunks per token row.
-  constexpr int CPR = KV8 ? D / 16 : D / 8;      // 16-byte chunks per row
-  constexpr int NL = BN * CPR / 128;             // chunks per thread (K and V each)
-  __shared__ unsigned char s_valid[BN];
-  uint4 kreg[NL], vreg[NL];
-  float ksc[NL], vsc[NL];
-  auto prefetch = [&](int j0) {
-#pragma unroll
-    for (int u = 0; u < NL; ++u) {
-      const int idx = tid + u * 128;
-      const int r = idx / CPR, c = idx % CPR;
-      const int j = j0 + r;
-      kreg[u] = make_uint4(0, 0, 0, 0);
-      vreg[u] = make_uint4(0, 0, 0, 0);
-      ksc[u] = -1.0f;  // marks an absent row
-      vsc[u] = 1.0f;
-      if (j < j_end) {
-        const int blk = checked_page(bt[j / a.page], a.num_blocks);
-        if (blk >= 0) {
-          const size_t row = ((size_t)blk * a.Hkv + kvh) * a.page + (j % a.page);
-          const size_t off = row * D * (KV8 ? 1 : 2) + (size_t)c * 16;
-          kreg[u] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(a.k_cache) + off));
-          vreg[u] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(a.v_cache) + off));
-          ksc[u] = (KV8 && a.k_scale) ? __ldg(a.k_scale + row) : 1.0f;
-          vsc[u] = (KV8 && a.v_scale) ? __ldg(a.v_scale + row) : 1.0f;
-        }
-      }
-    }
-  };
-  if (j_begin < j_end) prefetch(j_begin);
-  for (int j0 = j_begin; j0 < j_end; j0 += BN) {
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < NL; ++u) {
-      const int idx = tid + u * 128;
-      const int r = idx / CPR, c = idx % CPR;
-      const bool present = ksc[u] >= 0.0f;
-      if (c == 0) s_valid[r] = present ? 1 : 0;
-      if (KV8) {
-        const unsigned short* kp = reinterpret_cast<const unsigned short*>(&kreg[u]);
-        const unsigned short* vp = reinterpret_cast<const unsigned short*>(&vreg[u]);
-        uint4 ko[2], vo[2];
-        uint32_t* kw = reinterpret_cast<uint32_t*>(ko);
-        uint32_t* vw = reinterpret_cast<uint32_t*>(vo);
-        const float ks = present ? ksc[u] : 0.0f, vs = vsc[u];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float2 kk = fp8x2_to_float2(kp[e]);
-          const float2 vv = fp8x2_to_float2(vp[e]);
-          kw[e] = pack_bf16(kk.x * ks, kk.y * ks);
-          vw[e] = pack_bf16(vv.x * vs, vv.y * vs);
-        }
-        *reinterpret_cast<uint4*>(Ks + r * LDS + c * 16) = ko[0];
-        *reinterpret_cast<uint4*>(Ks + r * LDS + c * 16 + 8) = ko[1];
-        *reinterpret_cast<uint4*>(Vs + r * LDS + c * 16) = vo[0];
-        *reinterpret_cast<uint4*>(Vs + r * LDS + c * 16 + 8) = vo[1];
+  int ahead = j_begin;                                             // first token of the step that is requested next
+  int page_at = ahead / a.page, page_off = ahead - page_at * a.page;
+  int to = 0;                                                      // and the ring stage that it goes to
+  uint32_t there = 0;                                              // one bit per step under way: its page exists
+  auto request = [&](int place) {
+    if (ahead >= j_end) return;
+    const int blk = checked_page(bt[page_at], a.num_blocks);
+    there |= (uint32_t)(blk >= 0) << place;
+    if (elect_one()) {
+      uint64_t* bar = &bars[warp][to];
+      if (blk < 0) {
+        mbar_arrive(bar);
       } else {
-        *reinterpret_cast<uint4*>(Ks + r * LDS + c * 8) = kreg[u];
-        *reinterpret_cast<uint4*>(Vs + r * LDS + c * 8) = vreg[u];
+        const long long row = ((long long)blk * a.Hkv + kvh) * a.page + page_off;
+        uint8_t* st = ring + to * Shape::STEP_BYTES;
+        mbar_expect_tx(bar, 2 * Shape::ROWS_BYTES + (KV8 && a.k_scale ? 64 : 0) + (KV8 && a.v_scale ? 64 : 0));
+#pragma unroll
+        for (int c = 0; c < ATOMS; ++c) tma_load_2d(st + c * 2048, &tmK, bar, c * 64, (int)row);
+        if (KV8 && a.k_scale) bulk_load(scale_ring + to * 32, a.k_scale + row, 64, bar);
+        if (KV8 && a.v_scale) bulk_load(scale_ring + to * 32 + 16, a.v_scale + row, 64, bar);
+#pragma unroll
+        for (int c = 0; c < ATOMS; ++c) tma_load_2d(st + Shape::ROWS_BYTES + c * 2048, &tmV, bar, c * 64, (int)row);
       }
     }
-    __syncthreads();
-    if (j0 + BN < j_end) prefetch(j0 + BN);
-    const int tok0 = warp * 16;  // this warp's 16 tokens of the tile
-    if (j0 + tok0 >= j_end) continue;
+    __syncwarp();
+    if (++to == STAGES) to = 0;
+    ahead += SPAN;
+    for (page_off += SPAN; page_off >= a.page; page_off -= a.page) ++page_at;
+  };
+#pragma unroll
+  for (int i = 0; i < STAGES - 1; ++i) request(i);
+
+  // Q as the other operand, heads as columns: depth pairs (2 t4, 2 t4 + 1) and (+ 8, + 9) of a step for bf16, four consecutive
+  // elements 4 t4 .. 4 t4 + 3 for 8-bit rows
+  uint32_t qf[KT][2];
+  {
+    const bf16* q = a.q + ((size_t)b * a.Hq + (size_t)kvh * G + min(g, G - 1)) * D + (KV8 ? 4 : 2) * t4;
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+      qf[k][0] = *reinterpret_cast<const uint32_t*>(q + k * 16);
+      qf[k][1] = *reinterpret_cast<const uint32_t*>(q + k * 16 + (KV8 ? 2 : 8));
+      if (g >= G) qf[k][0] = qf[k][1] = 0;
+    }
+  }
+  float o[KT][4];
+#pragma unroll
+  for (int i = 0; i < KT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // heads 2 t4 and 2 t4 + 1; sums of this lane's tokens
+  const float sl2 = a.scale * 1.4426950408889634f;
+  constexpr float RAISE = 8.0f;
+  // Address of row r, 16-byte column c of 16 swizzled rows.  ldmatrix: lanes 8 i .. 8 i + 7 give the rows of matrix i.
+  auto cell = [](uint32_t base, int r, int c) { return base + (c >> 3) * 2048 + r * 128 + (((c & 7) ^ (r & 7)) << 4); };
+  const int lr = (lane & 7) + (lane & 8), lc = lane >> 4;            // K: matrices = tokens 0-7, 8-15 of a column, then of the next
+  const int vr = (lane & 7) + ((lane >> 1) & 8), vcol = (lane >> 3) & 1;  // V: matrices = columns c, c + 1 of tokens 0-7, then 8-15
+
+  int at = 0;              // ring stage of the step at work
+  uint32_t parity = 0;
+  bool ok = true;
+  for (int j = j_begin; j < j_end; j += SPAN) {
+    request(STAGES - 1);   // into the stage that the step before this one has left
+    ok = __all_sync(0xffffffffu, mbar_wait(&bars[warp][at], parity, 61));
+    if (!ok) break;
+    const uint32_t ks_at = smem_u32(ring + at * Shape::STEP_BYTES), vs_at = ks_at + Shape::ROWS_BYTES;
+    const float* scales = scale_ring + at * 32;
+    if (++at == STAGES) at = 0, parity ^= 1;
+    const bool page_there = there & 1;
+    there >>= 1;
+    if (!page_there) continue;
+    const int left = j_end - j;   // tokens of this step that exist, if fewer than 16
+    // S: tokens g and g + 8 (rows), heads 2 t4 and 2 t4 + 1 (columns)
     float s[2][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
+    for (int e = 0; e < 4; ++e) s[0][e] = s[1][e] = 0.0f;
+    if (KV8) {
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      uint32_t kb[4];
-      const int n = tok0 + (lane & 7) + 8 * (lane >> 4);
-      const int c = kk * 16 + 8 * ((lane >> 3) & 1);
-      ldsm_x4(kb, smem_u32(Ks + n * LDS + c));
-      mma_bf16(s[0], qf[kk], kb[0], kb[1]);
-      mma_bf16(s[1], qf[kk], kb[2], kb[3]);
-    }
-    // only row g (c0, c1 of each n-tile) is a real query head; rows g + 8 are padding
-    float mx = -INFINITY;
-    float p[2][2];
+      for (int k = 0; k < KT; k += 2) {   // a 16-byte column is one depth step
+        uint32_t x[4];
+        ldsm_x4(x, cell(ks_at, lr, k + lc));
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t f[4] = {fp8x2_to_bf16x2(x[2 * h] & 0xffff), fp8x2_to_bf16x2(x[2 * h + 1] & 0xffff), fp8x2_to_bf16x2(x[2 * h] >> 16),
+                                 fp8x2_to_bf16x2(x[2 * h + 1] >> 16)};
+          mma_bf16(s[h], f, qf[k + h][0], qf[k + h][1]);
+        }
+      }
+    } else {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const bool ok = s_valid[tok0 + i * 8 + t4 * 2 + e] != 0;
-        const float v = ok ? s[i][e] * sl2 : -INFINITY;
-        p[i][e] = v;
-        mx = fmaxf(mx, v);
+      for (int k = 0; k < KT; ++k) {
+        uint32_t f[4];
+        ldsm_x4(f, cell(ks_at, lr, 2 * k + lc));
+        mma_bf16(s[k & 1], f, qf[k][0], qf[k][1]);
       }
     }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float mn = fmaxf(m_run, mx);
-    const float m_use = (mn == -INFINITY) ? 0.0f : mn;
-    const float corr = (m_run == -INFINITY) ? 0.0f : exp2f(m_run - m_use);
-    m_run = mn;
-    float rs = 0.0f;
+    float vs[2] = {1.0f, 1.0f}, sc[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int h = 0; h < 2; ++h) {
+      const float ks = KV8 && a.k_scale ? scales[g + 8 * h] : 1.0f;
+      if (KV8 && a.v_scale) vs[h] = scales[16 + g + 8 * h];
+      const bool seen = g + 8 * h < left;
+      if (!seen) vs[h] = 0.0f;
+      sc[2 * h] = seen ? (s[0][2 * h] + s[1][2 * h]) * (sl2 * ks) : -INFINITY;
+      sc[2 * h + 1] = seen ? (s[0][2 * h + 1] + s[1][2 * h + 1]) * (sl2 * ks) : -INFINITY;
+    }
+    const float mx[2] = {fmaxf(sc[0], sc[2]), fmaxf(sc[1], sc[3])};
+    if (__any_sync(0xffffffffu, mx[0] > m_run[0] + RAISE || mx[1] > m_run[1] + RAISE)) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        p[i][e] = exp2f(p[i][e] - m_use);
-        rs += p[i][e];
+      for (int h = 0; h < 2; ++h) {
+        float m = fmaxf(m_run[h], mx[h]);
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        const float corr = m_run[h] == -INFINITY ? 0.0f : ex2_fast(m_run[h] - m);
+        m_run[h] = m;
+        l_run[h] *= corr;
+#pragma unroll
+        for (int i = 0; i < KT; ++i) o[i][h] *= corr, o[i][2 + h] *= corr;
       }
     }
-    rs += __shfl_xor_sync(0xffffffffu, rs, 1);
-    rs += __shfl_xor_sync(0xffffffffu, rs, 2);
-    l_run = l_run * corr + rs;
+    float p[4];
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      o[i][0] *= corr;
-      o[i][1] *= corr;
+    for (int e = 0; e < 4; ++e) {
+      const float m = m_run[e & 1];
+      p[e] = ex2_fast(sc[e] - (m == -INFINITY ? 0.0f : m));
+      l_run[e & 1] += p[e];
+      if (KV8) p[e] *= vs[e >> 1];
     }
-    uint32_t pa[4];
-    pa[0] = pack_bf16(p[0][0], p[0][1]);
-    pa[1] = 0;  // rows g + 8
-    pa[2] = pack_bf16(p[1][0], p[1][1]);
-    pa[3] = 0;
+    const uint32_t p0 = movmatrix_trans(pack_bf16(p[0], p[1])), p1 = movmatrix_trans(pack_bf16(p[2], p[3]));
+    // Rows past the end hold whatever their page holds: a probability of zero does not remove an infinity or NaN, so V is zeroed.
+    uint32_t keep[2] = {~0u, ~0u};
+    if (left < STEP) {
 #pragma unroll
-    for (int dp = 0; dp < D / 16; ++dp) {
-      uint32_t vb[4];
-      const int tok = tok0 + (lane & 7) + 8 * ((lane >> 3) & 1);
-      const int d = dp * 16 + 8 * (lane >> 4);
-      ldsm_x4_t(vb, smem_u32(Vs + tok * LDS + d));
-      mma_bf16(o[2 * dp], pa, vb[0], vb[1]);
-      mma_bf16(o[2 * dp + 1], pa, vb[2], vb[3]);
+      for (int h = 0; h < 2; ++h) keep[h] = (2 * t4 + 8 * h < left ? 0xffffu : 0u) | (2 * t4 + 1 + 8 * h < left ? 0xffff0000u : 0u);
     }
+    // O^T += V^T P^T.  bf16: rows g and g + 8 of tile i are elements 16 i + g and 16 i + 8 + g; 8-bit: 16 i + 2 g and 16 i + 2 g + 1
+    if (KV8) {
+#pragma unroll
+      for (int i = 0; i < KT; i += 2) {
+        uint32_t x[4];  // (column i, tokens 0-7), (i + 1, 0-7), (i, 8-15), (i + 1, 8-15): elements 2 g, 2 g + 1 of tokens 2 t4, 2 t4 + 1
+        ldsm_x4_t(x, cell(vs_at, vr, i + vcol));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t lo = x[h] & keep[0], hi = x[2 + h] & keep[1];
+          const uint32_t lo2 = __byte_perm(lo, 0, 0x3120), hi2 = __byte_perm(hi, 0, 0x3120);
+          const uint32_t f[4] = {fp8x2_to_bf16x2(lo2 & 0xffff), fp8x2_to_bf16x2(lo2 >> 16), fp8x2_to_bf16x2(hi2 & 0xffff), fp8x2_to_bf16x2(hi2 >> 16)};
+          mma_bf16(o[i + h], f, p0, p1);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < KT; ++i) {
+        uint32_t f[4];
+        ldsm_x4_t(f, cell(vs_at, vr, 2 * i + vcol));
+        f[0] &= keep[0], f[1] &= keep[0], f[2] &= keep[1], f[3] &= keep[1];
+        mma_bf16(o[i], f, p0, p1);
+      }
+    }
+    __syncwarp();  // every lane has read the stage before it is asked for again
   }
-  // merge the four warps (rows g < G only), reusing the tile buffers
+  if (!ok) {       // a wait ran out (recorded): copies under way land before shared memory is used again
+    for (int i = 0; i < STAGES; ++i)
+      if (there >> i & 1) (void)mbar_wait(&bars[warp][(at + i) % STAGES], parity ^ (at + i >= STAGES), 62);
+  }
+  // merge the four warps; their rings become the accumulators' place
   __syncthreads();
-  float* s_m = reinterpret_cast<float*>(Ks);          // [NWARP][G]
-  float* s_l = s_m + NWARP * G;                        // [NWARP][G]
-  float* s_acc = s_l + NWARP * G;                      // [NWARP][G][D]
-  if (g < G) {
-    if (t4 == 0) {
-      s_m[warp * G + g] = m_run;
-      s_l[warp * G + g] = l_run;
-    }
+  float* const s_acc = reinterpret_cast<float*>(dsm);  // [NWARP][8][D]
+  float* const b_acc = s_acc + NWARP * 8 * D;          // [8][D]
+  __shared__ float b_m[8], b_l[8];
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      s_acc[(warp * G + g) * D + i * 8 + t4 * 2] = o[i][0];
-      s_acc[(warp * G + g) * D + i * 8 + t4 * 2 + 1] = o[i][1];
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], d);
+    const int head = 2 * t4 + h;
+    if (head < G) {
+      if (g == 0) {
+        s_m[warp][head] = m_run[h];
+        s_l[warp][head] = l_run[h];
+      }
+#pragma unroll
+      for (int i = 0; i < KT; ++i) {
+        float* acc = s_acc + (warp * 8 + head) * D + i * 16;
+        if (KV8) {
+          *reinterpret_cast<float2*>(acc + 2 * g) = make_float2(o[i][h], o[i][2 + h]);
+        } else {
+          acc[g] = o[i][h];
+          acc[g + 8] = o[i][2 + h];
+        }
+      }
     }
   }
   __syncthreads();
@@ -780,17 +856,20 @@ __global__ void __launch_bounds__(128) paged_decode_mma_kernel(const DecodeArgs 
     const int gg = idx / D, d = idx % D;
     float mm = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < NWARP; ++w) mm = fmaxf(mm, s_m[w * G + gg]);
+    for (int w = 0; w < NWARP; ++w) mm = fmaxf(mm, s_m[w][gg]);
     float ll = 0.0f, oo = 0.0f;
 #pragma unroll
     for (int w = 0; w < NWARP; ++w) {
-      const float ms = s_m[w * G + gg];
-      const float c = (ms == -INFINITY) ? 0.0f : exp2f(ms - mm);
-      ll += s_l[w * G + gg] * c;
-      oo += s_acc[(w * G + gg) * D + d] * c;
+      const float ms = s_m[w][gg];
+      const float c = (ms == -INFINITY) ? 0.0f : ex2_fast(ms - mm);
+      ll += s_l[w][gg] * c;
+      oo += s_acc[(w * 8 + gg) * D + d] * c;
     }
     const int hq = kvh * G + gg;
-    if (a.nsplit == 1) {
+    if (a.clustered) {
+      b_acc[gg * D + d] = oo;
+      if (d == 0) b_m[gg] = mm, b_l[gg] = ll;
+    } else if (used == 1) {
       a.out[((size_t)b * a.Hq + hq) * D + d] = __float2bfloat16_rn(ll > 0.0f ? oo / ll : 0.0f);
     } else {
       // partial format shared with the SIMT kernel: natural-log domain maximum
@@ -802,25 +881,43 @@ __global__ void __launch_bounds__(128) paged_decode_mma_kernel(const DecodeArgs 
       }
     }
   }
-  if (a.nsplit == 1 || a.counters == nullptr) return;
+  if (a.clustered) {
+    cluster_sync_all();  // every split's sums are there; the output rows are shared out over the blocks
+    for (int idx = split * 128 + tid; idx < G * D; idx += 128 * a.nsplit) {
+      const int gg = idx / D;
+      float mm = -INFINITY, ll = 0.0f, oo = 0.0f;
+#pragma unroll 8
+      for (int r = 0; r < used; ++r) mm = fmaxf(mm, ld_cluster(cluster_addr(&b_m[gg], r)));
+#pragma unroll 8
+      for (int r = 0; r < used; ++r) {
+        const float ms = ld_cluster(cluster_addr(&b_m[gg], r));
+        const float c = (ms == -INFINITY) ? 0.0f : ex2_fast(ms - mm);
+        ll += ld_cluster(cluster_addr(&b_l[gg], r)) * c;
+        oo += ld_cluster(cluster_addr(&b_acc[idx], r)) * c;
+      }
+      a.out[((size_t)b * a.Hq + (size_t)kvh * G) * D + idx] = __float2bfloat16_rn(ll > 0.0f ? oo / ll : 0.0f);
+    }
+    cluster_sync_all();  // no block leaves while another still reads its sums
+    return;
+  }
+  if (used == 1 || a.counters == nullptr) return;
   __shared__ int s_last2;
   __threadfence();
   __syncthreads();
   if (tid == 0) {
     const int old = atomicAdd(&a.counters[b * a.Hkv + kvh], 1);
-    s_last2 = (old == a.nsplit - 1);
+    s_last2 = (old == used - 1);
     if (s_last2) a.counters[b * a.Hkv + kvh] = 0;
   }
   __syncthreads();
   if (!s_last2) return;
   __threadfence();
-  __shared__ float s_coef2[G][32];
-  __shared__ float s_inv2[G];
-  const int ns = a.nsplit;
+  __shared__ float s_coef2[8][32];
+  __shared__ float s_inv2[8];
   for (int gg = warp; gg < G; gg += NWARP) {
     const size_t bh = (size_t)b * a.Hq + kvh * G + gg;
-    const float ms = lane < ns ? __ldcg(&a.part_ml[(bh * ns + lane) * 2]) : -INFINITY;
-    const float ls = lane < ns ? __ldcg(&a.part_ml[(bh * ns + lane) * 2 + 1]) : 0.0f;
+    const float ms = lane < used ? __ldcg(&a.part_ml[(bh * a.nsplit + lane) * 2]) : -INFINITY;
+    const float ls = lane < used ? __ldcg(&a.part_ml[(bh * a.nsplit + lane) * 2 + 1]) : 0.0f;
     const float mm = warp_max(ms);
     const float c = (ms == -INFINITY) ? 0.0f : __expf(ms - mm);
     const float ll = warp_sum(ls * c);
@@ -831,10 +928,10 @@ __global__ void __launch_bounds__(128) paged_decode_mma_kernel(const DecodeArgs 
   for (int idx = tid; idx < G * D; idx += 128) {
     const int gg = idx / D, d = idx % D;
     const size_t bh = (size_t)b * a.Hq + kvh * G + gg;
-    const float* po = a.part_o + bh * ns * D + d;
+    const float* po = a.part_o + bh * a.nsplit * D + d;
     float oo = 0.0f;
 #pragma unroll 8
-    for (int sidx = 0; sidx < ns; ++sidx) oo += __ldcg(po + (size_t)sidx * D) * s_coef2[gg][sidx];
+    for (int sidx = 0; sidx < used; ++sidx) oo += __ldcg(po + (size_t)sidx * D) * s_coef2[gg][sidx];
     a.out[bh * D + d] = __float2bfloat16_rn(oo * s_inv2[gg]);
   }
 }
@@ -872,28 +969,43 @@ int dispatch_flash(const FlashArgs& a, int hd, int max_q_len, int S, cudaStream_
   return -2;
 }
 
-template <int D, int G, bool KV8>
+// The tensor-core kernel copies whole 16-token steps of 16-byte vectors.
+bool decode_mma_fits(const DecodeArgs& a, int D) {
+  const unsigned long long addr = reinterpret_cast<unsigned long long>(a.k_cache) | reinterpret_cast<unsigned long long>(a.v_cache) |
+                                  reinterpret_cast<unsigned long long>(a.k_scale) | reinterpret_cast<unsigned long long>(a.v_scale);
+  return a.page % 16 == 0 && (addr & 15) == 0 && (reinterpret_cast<unsigned long long>(a.q) & 3) == 0 && a.num_blocks > 0 &&
+         (long long)a.num_blocks * a.Hkv * a.page < (1ll << 31);
+}
+template <int D, bool KV8>
 int launch_decode_mma(const DecodeArgs& a, int B, cudaStream_t stream, bool pdl) {
-  const size_t smem = (size_t)(16 + 2 * 64) * (D + 8) * sizeof(bf16);
-  static bool configured = false;
-  if (!configured && smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel<D, G, KV8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  return (int)prism_launch(paged_decode_mma_kernel<D, G, KV8>, dim3(B, a.Hkv, a.nsplit), dim3(128), smem, stream, pdl, a);
+  constexpr int smem = DecodeShape<D, KV8>::SMEM_BYTES;
+  static const cudaError_t configured = [] {
+    cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }();
+  if (configured != cudaSuccess) return (int)configured;
+  // 8-bit rows are described as half as many 16-bit elements: the copy only moves bytes
+  const unsigned long long rows = (unsigned long long)a.num_blocks * a.Hkv * a.page, cols = KV8 ? D / 2 : D;
+  CUtensorMap tk, tv;
+  int rc = prism_get_tensor_map(a.k_cache, rows, cols, cols, 16, &tk);
+  if (rc == 0) rc = prism_get_tensor_map(a.v_cache, rows, cols, cols, 16, &tv);
+  if (rc) return rc;
+  DecodeArgs c = a;
+  c.clustered = a.counters != nullptr && (a.nsplit == 2 || a.nsplit == 4 || a.nsplit == 8 || a.nsplit == 16);
+  return (int)prism_launch_clusters(paged_decode_mma_kernel<D, KV8>, dim3(B, a.Hkv, a.nsplit), dim3(128), smem, stream, pdl,
+                                    c.clustered ? a.nsplit : 1, tk, tv, c);
 }
 
 // use_mma: tensor-core kernel (larger batches); otherwise the SIMT kernel (lowest latency at batch 1)
 template <int D, bool KV8>
 int dispatch_decode(const DecodeArgs& a, int B, cudaStream_t stream, bool pdl, bool use_mma) {
   dim3 grid(B, a.Hkv, a.nsplit), block(128);
-  if (use_mma) {
+  if (use_mma && decode_mma_fits(a, D)) {
     switch (a.Hq / a.Hkv) {
-      case 1: return launch_decode_mma<D, 1, KV8>(a, B, stream, pdl);
-      case 2: return launch_decode_mma<D, 2, KV8>(a, B, stream, pdl);
-      case 4: return launch_decode_mma<D, 4, KV8>(a, B, stream, pdl);
-      case 8: return launch_decode_mma<D, 8, KV8>(a, B, stream, pdl);
+      case 1:
+      case 2:
+      case 4:
+      case 8: return launch_decode_mma<D, KV8>(a, B, stream, pdl);
     }
     return -3;
   }
@@ -936,6 +1048,7 @@ PRISM_API int prism_paged_decode(const void* q, const void* k_cache, const void*
   a.num_blocks = num_blocks;
   a.nsplit = nsplit < 1 ? 1 : (nsplit > 32 ? 32 : nsplit);
   a.scale = scale;
+  a.clustered = 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int rc;
   const bool mma = use_mma != 0;

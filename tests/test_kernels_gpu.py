@@ -559,3 +559,37 @@ def test_gemm_on_sm_pairs(cuda_device, T, M, K, form):
     tol = 2.0 * 4.0 * (K / 16 + 16) * 2.0 ** -23 if got.dtype == torch.float32 else 1.2e-2
     err = (got.double().cpu() - want).abs() / (1.0 + want.abs())
     assert err.max() < tol, (form, err.max())
+
+
+@pytest.mark.parametrize("mode", [ops.KV_BF16, ops.KV_FP8_SCALED])
+@pytest.mark.parametrize("D,G,page", [(128, 8, 16), (128, 1, 32), (64, 2, 64), (64, 8, 24)])
+@pytest.mark.parametrize("nsplit", [1, 3, 8, 16])
+def test_paged_decode_steps_holes_and_stale_rows(cuda_device, mode, D, G, page, nsplit):
+    """Contexts around the 16-token step and the 64-token span, a hole inside one, pages that are not whole steps, and NaN in rows that
+    no context reaches: they share pages with rows that are read."""
+    Hkv, blocks, maxblk = 2, 64, 12
+    cg, cc = _fill_cache(mode, 1, blocks, Hkv, page, D, seed=81)
+    ctx = torch.tensor([1, 15, 16, 17, 63, 65, 129, 0, 9 * page - 3, 11 * page + 1], dtype=torch.int32).clamp(max=maxblk * page)
+    bt = torch.full((len(ctx), maxblk), -1, dtype=torch.int32)
+    used = 0
+    for b, n in enumerate(ctx.tolist()):
+        pages = -(-n // page)
+        bt[b, :pages] = torch.arange(pages, dtype=torch.int32) + used % 20
+        used += 3
+    bt[8, 4] = -1
+    seen = torch.zeros(blocks * page, dtype=torch.bool)
+    for b, n in enumerate(ctx.tolist()):
+        for t in range(n):
+            if bt[b, t // page] >= 0:
+                seen[int(bt[b, t // page]) * page + t % page] = True
+    stale = (~seen).view(blocks, 1, page).expand(-1, Hkv, -1).cuda()
+    payload = cg.payload.view(torch.uint8) if mode != ops.KV_BF16 else cg.payload
+    for kv in (0, 1):
+        payload[kv, 0][stale] = 0x7F if mode != ops.KV_BF16 else float("nan")
+        if cg.scales is not None:
+            cg.scales[kv, 0][stale] = float("nan")
+    q = rand_bf16(len(ctx), G * Hkv, D, seed=82)
+    yg = ops.paged_decode_attention(q.cuda(), cg, 0, bt.cuda(), ctx.cuda(), nsplit=nsplit, use_mma=True)
+    yc = ops.paged_decode_attention(q.float(), cc, 0, bt, ctx)
+    err = (yg.float().cpu() - yc).abs()
+    assert err.max() < 2e-2 and err.mean() < 2e-3, (err.max(), err.mean())
