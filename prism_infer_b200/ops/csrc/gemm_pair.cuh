@@ -11,9 +11,11 @@
 // gated 344 -> 266 us (1548 TFLOP/s, the power limit's rate), 7500 tokens 1296 -> 952; 1616 x 12288 -> 4096 177 -> 133; 6272 x 1152
 // -> 4304 with GELU 60 -> 51; 230 x 4096 -> 6144 33 -> 18.
 //
-// Tokens lie on the TMEM lanes, so a thread of the epilogue owns one token row and moves bias, residual and output as 16-byte
-// vectors.  Eight epilogue warps (two per lane quarter) drain one accumulator while the next tile fills the other; each asks for its next
-// residual vectors before it works on the present ones.
+// Tokens lie on the TMEM lanes, so a thread of the epilogue gets 16 features of one token row at a time.  Eight epilogue warps (two
+// per lane quarter) drain one accumulator while the next tile fills the other.  bf16 results turn in shared memory (32 rows x 64
+// features a warp, columns XORed with the row against bank conflicts) and leave, with the residual, as whole 128-byte lines: lanes
+// that store 16 bytes each into 32 rows cost 32 requests to L2 per instruction, and short products were bound by them (6272 x 1152 -> 3456
+// with bias: 61 -> 51 us; 1152 -> 1152 with bias and residual: 35 -> 26).
 //
 // The TMA loads carry cta_group::2 only so that both CTAs' copies may report to the even CTA's barrier; none is multicast.
 #pragma once
@@ -22,6 +24,7 @@
 
 constexpr int PAIR_THREADS = 320;           // producer warp, MMA warp, eight epilogue warps
 constexpr int PAIR_EPI_WARPS = 8;
+constexpr int PAIR_TURN_BYTES = PAIR_EPI_WARPS * 4096;
 constexpr int PAIR_GROUP = 8;               // token tiles (of 256) walked before the next feature tile
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
@@ -80,16 +83,13 @@ struct PairArgs {
   PrismSections sec;
 };
 
-__device__ __forceinline__ void add_bf16x16(float (&v)[16], const uint4& r0, const uint4& r1, bool round_first) {
-  const __nv_bfloat162* p0 = reinterpret_cast<const __nv_bfloat162*>(&r0);
-  const __nv_bfloat162* p1 = reinterpret_cast<const __nv_bfloat162*>(&r1);
+__device__ __forceinline__ void add_bf16x8(float* v, const uint4& x) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&x);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const float2 x0 = __bfloat1622float2(p0[e]), x1 = __bfloat1622float2(p1[e]);
-    v[2 * e] = (round_first ? bf16_round(v[2 * e]) : v[2 * e]) + x0.x;
-    v[2 * e + 1] = (round_first ? bf16_round(v[2 * e + 1]) : v[2 * e + 1]) + x0.y;
-    v[8 + 2 * e] = (round_first ? bf16_round(v[8 + 2 * e]) : v[8 + 2 * e]) + x1.x;
-    v[9 + 2 * e] = (round_first ? bf16_round(v[9 + 2 * e]) : v[9 + 2 * e]) + x1.y;
+    const float2 f = __bfloat1622float2(p[e]);
+    v[2 * e] += f.x;
+    v[2 * e + 1] += f.y;
   }
 }
 
@@ -102,7 +102,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   const int stages = a.stages;
   const int b_bytes = a.bn * 64;                       // bn / 2 rows of 128 bytes
   const int stage_bytes = A_BYTES + b_bytes;           // a multiple of 2 KB
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)stages * stage_bytes);  // the even CTA's are the ones in use
+  uint8_t* const turns = smem + (size_t)stages * stage_bytes;                          // [8] 32 rows of 128 bytes
+  uint64_t* full = reinterpret_cast<uint64_t*>(turns + PAIR_TURN_BYTES);               // the even CTA's are the ones in use
   uint64_t* empty = full + stages;
   uint64_t* acc_full = empty + stages;                 // [2] MMA -> the epilogues of both CTAs
   uint64_t* acc_empty = acc_full + 2;                  // [2] both epilogues -> MMA; the even CTA's are the ones in use
@@ -218,89 +219,114 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   } else {
     // ------------------------------ epilogue warps 2..9 ------------------------------
     const int q = warp & 3, half = (warp - 2) >> 2;  // TMEM lane quarter this warp may read; which half of the columns
+    uint4* const turn = reinterpret_cast<uint4*>(turns + (warp - 2) * 4096);
     pdl_wait();
     int local = 0;
     for (int tile = pair; tile < num_tiles; tile += pairs, ++local) {
       const int buf = local & 1;
       int m0, n0, kb0, kb1;
       tile_at(tile, m0, n0, kb0, kb1);
-      const int m = m0 + (int)rank * 128 + q * 32 + lane;
-      const bool m_ok = m < a.T;
-      // columns of this warp: outputs f0 + [c_lo, c_hi)
-      const int width = a.dual ? a.bn / 2 : a.bn, f0 = a.dual ? n0 / 2 : n0;
-      const int c_lo = half * (width / 2), c_hi = min(c_lo + width / 2, (a.dual ? a.N / 2 : a.N) - f0);
-      const uint4* rs = (a.residual != nullptr && m_ok) ? reinterpret_cast<const uint4*>(a.residual + (size_t)m * a.ldr + f0) : nullptr;
-      uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
-      if (rs != nullptr && c_lo < c_hi) {
-        r0 = rs[c_lo / 8];
-        r1 = rs[c_lo / 8 + 1];
-      }
+      // outputs of this tile: f0 + [0, width); the two warps of a lane quarter take half of the columns each, up to 64 at a time
+      const int f0 = a.dual ? n0 / 2 : n0, full_width = a.dual ? a.bn / 2 : a.bn, width = min(full_width, (a.dual ? a.N / 2 : a.N) - f0);
+      const int u_end = min(width, (half + 1) * (full_width / 2));
+      const int row0 = m0 + (int)rank * 128 + q * 32;  // first token of this warp
       if (!mbar_wait(&acc_full[buf], (uint32_t)(local >> 1) & 1, 3)) break;
       tc_fence_after();
       const uint32_t t_lane = tmem_base + buf * BUF_COLS + ((uint32_t)(q * 32) << 16);
-      for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
-        uint32_t r[16];
-        float v[16];
-        tmem_ld16(t_lane + c0, r);
-        if (a.dual) {
-          uint32_t ru[16];
-          tmem_ld16(t_lane + width + c0, ru);
-          tmem_ld_wait();
+      for (int u0 = half * (full_width / 2); u0 < u_end; u0 += 64) {
+        // the unit's residual, in the order in which it will be stored
+        uint4 res[8];
+        const int u1 = min(u0 + 64, u_end), cu = u0 + (lane & 7) * 8;  // cu: first of the eight columns that this lane stores
+        if (a.residual != nullptr) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = glu(__uint_as_float(r[j]), __uint_as_float(ru[j]), a.act, a.glu_limit);
-        } else {
-          const int f = f0 + c0;
-          int act = a.act;
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-          if (a.sec.n > 0) {
-            float alpha;
-            prism_section_of(a.sec, f, alpha, act);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] *= alpha;
-          }
-          if (a.bias != nullptr) {
-            const uint4* b = reinterpret_cast<const uint4*>(a.bias + f);
-            add_bf16x16(v, b[0], b[1], false);
-          }
-          if (act == PRISM_ACT_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gelu_tanh(v[j]);
-          } else if (act == PRISM_ACT_GELU_ERF) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = gelu_erf(v[j]);
-          } else if (act == PRISM_ACT_SIGMOID) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = sigmoid_fast(v[j]);
-          } else if (act == PRISM_ACT_DECAY) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = decay_of(v[j]);
-          }
-          if (rs != nullptr) {
-            const uint4 x0 = r0, x1 = r1;
-            if (c0 + 16 < c_hi) {
-              r0 = rs[c0 / 8 + 2];
-              r1 = rs[c0 / 8 + 3];
-            }
-            add_bf16x16(v, x0, x1, true);
+          for (int i = 0; i < 8; ++i) {
+            const int m = row0 + i * 4 + (lane >> 3);
+            res[i] = m < a.T && cu < u1 ? *reinterpret_cast<const uint4*>(a.residual + (size_t)m * a.ldr + f0 + cu) : make_uint4(0, 0, 0, 0);
           }
         }
-        if (!m_ok) continue;
-        if (a.out_f32) {
-          float* slab = reinterpret_cast<float*>(a.out) + (a.splits == 1 ? 0 : (kb0 / a.kb_per_split) * a.split_stride);
-          float4* dst = reinterpret_cast<float4*>(slab + (size_t)m * a.ldo + f0 + c0);
+        for (int c0 = u0; c0 < u1; c0 += 16) {
+          uint32_t r[16];
+          float v[16];
+          tmem_ld16(t_lane + c0, r);
+          if (a.dual) {
+            uint32_t ru[16];
+            tmem_ld16(t_lane + a.bn / 2 + c0, ru);
+            tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-        } else {
+            for (int j = 0; j < 16; ++j) v[j] = glu(__uint_as_float(r[j]), __uint_as_float(ru[j]), a.act, a.glu_limit);
+          } else {
+            const int f = f0 + c0;
+            int act = a.act;
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+            if (a.sec.n > 0) {
+              float alpha;
+              prism_section_of(a.sec, f, alpha, act);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] *= alpha;
+            }
+            if (a.bias != nullptr) {
+              const uint4* b = reinterpret_cast<const uint4*>(a.bias + f);
+              add_bf16x8(&v[0], b[0]);
+              add_bf16x8(&v[8], b[1]);
+            }
+            if (act == PRISM_ACT_GELU_TANH) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = gelu_tanh(v[j]);
+            } else if (act == PRISM_ACT_GELU_ERF) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = gelu_erf(v[j]);
+            } else if (act == PRISM_ACT_SIGMOID) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = sigmoid_fast(v[j]);
+            } else if (act == PRISM_ACT_DECAY) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = decay_of(v[j]);
+            }
+          }
+          if (a.out_f32) {
+            if (row0 + lane < a.T) {
+              float* slab = reinterpret_cast<float*>(a.out) + (a.splits == 1 ? 0 : (kb0 / a.kb_per_split) * a.split_stride);
+              float4* dst = reinterpret_cast<float4*>(slab + (size_t)(row0 + lane) * a.ldo + f0 + c0);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+            }
+            continue;
+          }
           uint4 o[2];
           __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(o);
 #pragma unroll
           for (int e = 0; e < 8; ++e) op[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + f0 + c0);
-          dst[0] = o[0];
-          dst[1] = o[1];
+          const int c = (c0 - u0) / 8;
+          turn[lane * 8 + (c ^ (lane & 7))] = o[0];
+          turn[lane * 8 + ((c + 1) ^ (lane & 7))] = o[1];
         }
+        if (a.out_f32) continue;
+        __syncwarp();
+        if (cu < u1) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3), m = row0 + r;
+            uint4 o = turn[r * 8 + ((lane ^ r) & 7)];
+            if (a.residual != nullptr) {
+              float v[8];
+              const __nv_bfloat162* op = reinterpret_cast<const __nv_bfloat162*>(&o);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 x = __bfloat1622float2(op[e]);
+                v[2 * e] = x.x;
+                v[2 * e + 1] = x.y;
+              }
+              add_bf16x8(v, res[i]);
+              __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) wp[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+            }
+            if (m < a.T) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + (size_t)m * a.ldo + f0 + cu) = o;
+          }
+        }
+        __syncwarp();
       }
       // this warp's reads of the accumulator are complete: hand the buffer back
       tc_fence_before();

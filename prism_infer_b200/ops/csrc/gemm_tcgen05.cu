@@ -853,9 +853,9 @@ int launch_pair(const void* W, const void* X, int K, long long ldw, long long ld
   a.bn = pair_columns(a.m_tiles * a.splits, a.N, a.dual != 0);
   a.n_tiles = (a.N + a.bn - 1) / a.bn;
   const int stage_bytes = W_TILE_BYTES + a.bn * 64;
-  a.stages = (SMEM_LIMIT - 1024 - 512) / stage_bytes;
+  a.stages = (SMEM_LIMIT - 1024 - 512 - PAIR_TURN_BYTES) / stage_bytes;
   if (a.stages > 12) a.stages = 12;
-  const size_t smem = (size_t)a.stages * stage_bytes + 1024 + (2 * a.stages + 4) * 8 + 64;
+  const size_t smem = (size_t)a.stages * stage_bytes + PAIR_TURN_BYTES + 1024 + (2 * a.stages + 4) * 8 + 64;
   CUtensorMap tx, tw;
   int rc = get_tensor_map(X, (unsigned long long)a.T, (unsigned long long)K, (unsigned long long)ldx, 128, &tx);
   if (rc) return rc;
