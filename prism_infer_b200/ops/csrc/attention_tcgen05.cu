@@ -240,6 +240,10 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int last_key = pos_off + row;     // last key position this row sees under the causal mask
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const float sl2 = a.scale * 1.4426950408889634f;
+    // A positive scale keeps the order of the scores: it then joins the subtraction of the maximum in one multiply-add, two scores to an
+    // instruction (2048 queries over 16384 keys, 32 heads: 618 -> 605 us; the chain of a tile's hand-offs bounds it, not the issue rate).
+    const bool scaled_later = sl2 > 0.0f;
+    const float factor = scaled_later ? sl2 : 1.0f;
     constexpr int HC = FA_BN / 2;           // keys per thread and tile
     constexpr int HO = 64;                  // first output column of the second thread of a pair
     constexpr int CHUNKS = HD_PAD / 16;     // 16-column chunks of the accumulator
@@ -265,14 +269,23 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_ld_wait();
         }
 #pragma unroll
-        for (int i = 0; i < HC; ++i) s[i] = __uint_as_float(r[i]) * sl2;
+        for (int i = 0; i < HC; ++i) s[i] = __uint_as_float(r[i]);
+        if (!scaled_later) {
+#pragma unroll
+          for (int i = 0; i < HC; ++i) s[i] *= sl2;
+        }
         if (j0 + HC > kv_len || (a.causal && j0 + HC - 1 > last_key)) {
 #pragma unroll
           for (int i = 0; i < HC; ++i)
             if (j0 + i >= kv_len || (a.causal && j0 + i > last_key)) s[i] = -INFINITY;
         }
+        float mb = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < HC; ++i) mx = fmaxf(mx, s[i]);
+        for (int i = 0; i < HC; i += 4) {
+          mx = max3(mx, s[i], s[i + 1]);
+          mb = max3(mb, s[i + 2], s[i + 3]);
+        }
+        mx = fmaxf(mx, mb) * factor;
       }
       // pair maximum, and an OR over the CTA of "some row must raise its reference"
       mx_s[(b * 2 + half) * FA_BM + r_local] = mx;
@@ -305,16 +318,19 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
       const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
-      float sum = 0.0f;
       uint32_t packed[HC / 2];
+      const unsigned long long f2 = pair_of(factor, factor), m2 = pair_of(-m_use, -m_use);
+      unsigned long long sum[2] = {0, 0};
 #pragma unroll
       for (int i = 0; i < HC; i += 2) {
-        const float p0 = ex2f(s[i] - m_use), p1 = ex2f(s[i + 1] - m_use);
-        sum += p0 + p1;
+        const float2 x = unpair(fma2(pair_of(s[i], s[i + 1]), f2, m2));
+        const float p0 = ex2f(x.x), p1 = ex2f(x.y);
+        sum[(i >> 1) & 1] = add2(sum[(i >> 1) & 1], pair_of(p0, p1));
         __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
         packed[i >> 1] = *reinterpret_cast<uint32_t*>(&v);
       }
-      l_run += sum;
+      const float2 total = unpair(add2(sum[0], sum[1]));
+      l_run += total.x + total.y;
       tmem_st16(lane_addr + TMEM_S + b * FA_BN + half * (HC / 2), packed);
       tmem_st_wait();
       tc_fence_before();
