@@ -9,7 +9,7 @@
 // stage 400: 64-column tiles cost as much as 256-column ones.  With elect.sync and a carried stage a k-block is bound by its 512
 // tensor cycles (256 columns).  Measured, start -> now (single-SM form with feature or token rows before): 2048 x 4096 -> 2 x 12288
 // gated 344 -> 266 us (1548 TFLOP/s, the power limit's rate), 7500 tokens 1296 -> 952; 1616 x 12288 -> 4096 177 -> 133; 6272 x 1152
-// -> 4304 with GELU 60 -> 51; 230 x 4096 -> 6144 33 -> 18.
+// -> 4304 with GELU 60 -> 57; 230 x 4096 -> 6144 33 -> 19.
 //
 // Tokens lie on the TMEM lanes, so a thread of the epilogue gets 16 features of one token row at a time.  Eight epilogue warps (two
 // per lane quarter) drain one accumulator while the next tile fills the other.  bf16 results turn in shared memory (32 rows x 64
@@ -17,7 +17,8 @@
 // that store 16 bytes each into 32 rows cost 32 requests to L2 per instruction, and short products were bound by them (6272 x 1152 -> 3456
 // with bias: 61 -> 51 us; 1152 -> 1152 with bias and residual: 35 -> 26).
 //
-// The TMA loads carry cta_group::2 only so that both CTAs' copies may report to the even CTA's barrier; none is multicast.
+// The TMA loads carry cta_group::2 only so that both CTAs' copies may report to the even CTA's barrier; every copy goes to its own CTA.
+// MMA completion is reported to the even CTA, whose producer and epilogue pass it on to the odd one.
 #pragma once
 
 #include "common.cuh"
@@ -30,6 +31,11 @@ constexpr int PAIR_GROUP = 8;               // token tiles (of 256) walked befor
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
+// The same without ordering this thread's own accesses (a release at cluster scope took 1300 cycles behind TMA copies under way): for
+// passing on that a stage has been read.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 __device__ __forceinline__ void pair_tmem_alloc(uint32_t* smem_slot, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
 }
@@ -39,11 +45,33 @@ __device__ __forceinline__ void pair_tmem_relinquish() {
 __device__ __forceinline__ void pair_tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
 }
-// Arrives on the barrier at the same offset in BOTH CTAs once every MMA issued so far is done.
+// Arrives on this CTA's barrier once every MMA of the pair issued so far is done.
 __device__ __forceinline__ void pair_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"((uint16_t)3)
-               : "memory");
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// mbar_wait for a barrier on which the other CTA arrives.
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, int tag) {
+  auto done = [&] {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+  };
+  if (done()) return true;
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 128; ++i)
+      if (done()) return true;
+    if (clock64() - t0 > PRISM_WAIT_CYCLES) break;
+  }
+  prism_report(PRISM_ERR_MBAR_TIMEOUT, tag);
+  return false;
 }
 __device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -105,7 +133,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   uint8_t* const turns = smem + (size_t)stages * stage_bytes;                          // [8] 32 rows of 128 bytes
   uint64_t* full = reinterpret_cast<uint64_t*>(turns + PAIR_TURN_BYTES);               // the even CTA's are the ones in use
   uint64_t* empty = full + stages;
-  uint64_t* acc_full = empty + stages;                 // [2] MMA -> the epilogues of both CTAs
+  uint64_t* acc_full = empty + stages;                 // [2] MMA -> epilogue
   uint64_t* acc_empty = acc_full + 2;                  // [2] both epilogues -> MMA; the even CTA's are the ones in use
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
@@ -155,7 +183,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     if (elect_one()) {
       int s = 0, early = 0;        // ring stage; k-blocks whose weight tile is already under way
       uint32_t parity = 1;         // of the empty barrier: a fresh one counts as free
-      bool ok = true;
+      bool ok = true, reused = false;  // reused: the ring has gone round, its stages are free when the MMAs say so
       int m0, n0, kb0, kb1;
       tile_at(pair, m0, n0, kb0, kb1);
       // the first ring of weight tiles depends on no earlier kernel
@@ -170,12 +198,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
         tile_at(tile, m0, n0, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty[s], parity, 1);
+          ok = pair_wait(&empty[s], parity, 1);
           if (!ok) break;
+          if (rank == 0 && reused) mbar_arrive_cluster_relaxed(cluster_addr(&empty[s], 1));
           if (early < pre) ++early;
           else load_w(s, kb, n0);
           pair_tma_load_2d(smem + (size_t)s * stage_bytes, &tmX, cluster_addr(&full[s], 0), kb * 64, m0 + (int)rank * 128);
-          if (++s == stages) s = 0, parity ^= 1;
+          if (++s == stages) s = 0, parity ^= 1, reused = true;
         }
       }
       if (!ok && rank == 0) {
@@ -195,7 +224,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local) {
         const int buf = local & 1;
         if (local >= 2) {
-          ok = mbar_wait(&acc_empty[buf], ((uint32_t)(local >> 1) - 1) & 1, 5);
+          ok = pair_wait(&acc_empty[buf], ((uint32_t)(local >> 1) - 1) & 1, 5);
           if (!ok) break;
           tc_fence_after();
         }
@@ -230,8 +259,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       const int f0 = a.dual ? n0 / 2 : n0, full_width = a.dual ? a.bn / 2 : a.bn, width = min(full_width, (a.dual ? a.N / 2 : a.N) - f0);
       const int u_end = min(width, (half + 1) * (full_width / 2));
       const int row0 = m0 + (int)rank * 128 + q * 32;  // first token of this warp
-      if (!mbar_wait(&acc_full[buf], (uint32_t)(local >> 1) & 1, 3)) break;
+      if (!pair_wait(&acc_full[buf], (uint32_t)(local >> 1) & 1, 3)) break;
       tc_fence_after();
+      if (rank == 0 && warp == 2) {
+        tc_fence_before();
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_full[buf], 1));
+      }
       const uint32_t t_lane = tmem_base + buf * BUF_COLS + ((uint32_t)(q * 32) << 16);
       for (int u0 = half * (full_width / 2); u0 < u_end; u0 += 64) {
         // the unit's residual, in the order in which it will be stored
