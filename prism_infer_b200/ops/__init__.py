@@ -20,8 +20,6 @@ import torch.nn.functional as F
 
 from . import native
 
-_current_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
-
 KV_BF16, KV_FP8, KV_FP8_SCALED = 0, 1, 2
 FP8_MAX = 448.0
 FP8_SCALE_FLOOR = 1.0e-6
@@ -45,9 +43,9 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _s() -> int:
-    """Raw handle of the current device's current stream.  Asked for at every launch: the Python object of ``torch.cuda.current_stream()``
-    resolves its device anew each time, a third of the host time of a short prompt's step (230 tokens: 718 -> @@HOST@@ us a step)."""
-    return _current_raw_stream(_current_device())
+    """Raw handle of the current device's current stream, asked for at every launch.  The two functions exist only in builds of torch
+    with CUDA, so they are looked up here and not at import: the CPU statements of this module run without them."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _pdl() -> int:

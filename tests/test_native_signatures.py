@@ -4,6 +4,8 @@ prototypes in ``ops/csrc`` (a mismatch corrupts arguments silently)."""
 import glob
 import os
 import re
+import subprocess
+import sys
 
 from prism_infer_b200.ops import native
 
@@ -33,3 +35,18 @@ def test_no_cluster_qualified_bulk_loads_in_kernel_sources():
     banned = "multi" + "cast"
     for f in glob.glob(os.path.join(root, "*")):
         assert banned not in open(f).read(), f
+
+
+def test_ops_run_on_a_torch_without_cuda_bindings():
+    """A CPU build of torch has no ``torch._C._cuda_*`` functions: the op layer and its CPU statements do without them."""
+    code = (
+        "import torch\n"
+        "for name in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+        "    if hasattr(torch._C, name):\n"
+        "        delattr(torch._C, name)\n"
+        "from prism_infer_b200 import ops\n"
+        "x = torch.eye(8)\n"
+        "assert torch.equal(ops.linear(x, 2 * x), 2 * x)\n"
+    )
+    done = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=600)
+    assert done.returncode == 0, done.stderr
