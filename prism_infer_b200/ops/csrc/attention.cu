@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(BM * 2, MODE == 2 ? (BM == 128 ? 1 : 2) : (BM 
 }
 
 // =====================================================================================
-// Decode on the tensor cores (mma.sync m16n8k16), at most 8 query heads per KV head, pages of whole 16-token steps.  Same split-KV
+// Decode on the tensor cores (mma.sync m16n8k16), at most 8 query heads per KV head.  Same split-KV
 // partial format and in-kernel merge as the kernel above where the splits are not a cluster; the splits of a cluster read each other's
 // partial sums from shared memory instead (write, fence, count and read back through memory took 4 us of a 13 us call).
 //
@@ -631,7 +631,10 @@ struct DecodeShape {
   static constexpr int SMEM_BYTES = RING + SCALES + 1024;
 };
 
-template <int D, bool KV8>
+// WHOLE: pages are whole 16-token steps, one TMA box each.  Otherwise the lanes copy a step's rows, each from its own page, to the
+// same places: 16 sequences of 512 to 2048 tokens over pages of 24 take 20.1 us in bf16 and 23.7 in 8 bits (pages of 16 by TMA: 20.2 and
+// 23.4; the tile form 50 and 48; the SIMT kernel 136 and 76).
+template <int D, bool KV8, bool WHOLE>
 __global__ void __launch_bounds__(128, DecodeShape<D, KV8>::ATOMS == 2 ? 2 : 3)
 paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeArgs a) {
   using Shape = DecodeShape<D, KV8>;
@@ -647,7 +650,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   const int G = a.Hq / a.Hkv;
   uint8_t* const ring = dsm + warp * STAGES * Shape::STEP_BYTES;
   float* const scale_ring = reinterpret_cast<float*>(dsm + Shape::RING) + warp * STAGES * 32;
-  if (lane == 0) {
+  if (WHOLE && lane == 0) {
     for (int i = 0; i < STAGES; ++i) mbar_init(&bars[warp][i], 1);
     fence_barrier_init();
   }
@@ -667,7 +670,36 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   int page_at = ahead / a.page, page_off = ahead - page_at * a.page;
   int to = 0;                                                      // and the ring stage that it goes to
   uint32_t there = 0;                                              // one bit per step under way: its page exists
+  unsigned long long rows_there = 0;                               // or 16 of them: the rows that exist
+  // Address of row r, 16-byte column c of 16 swizzled rows.  ldmatrix: lanes 8 i .. 8 i + 7 give the rows of matrix i.
+  auto cell = [](uint32_t base, int r, int c) { return base + (c >> 3) * 2048 + r * 128 + (((c & 7) ^ (r & 7)) << 4); };
+  auto request_rows = [&](int place) {
+    if (ahead < j_end) {
+      constexpr int COLS = D * (KV8 ? 1 : 2) / 16;                 // 16-byte columns of a row
+      const int token = ahead + (lane & 15);
+      int blk = -1;
+      if (token < j_end) blk = checked_page(bt[token / a.page], a.num_blocks);
+      const long long row = blk < 0 ? 0 : ((long long)blk * a.Hkv + kvh) * a.page + token % a.page;
+      rows_there |= (unsigned long long)(__ballot_sync(0xffffffffu, blk >= 0) & 0xffff) << (16 * place);
+      uint8_t* const st = ring + to * Shape::STEP_BYTES;
+#pragma unroll
+      for (int i = 0; i < COLS / 2; ++i) {
+        const int r = (lane + 32 * i) / COLS, c = (lane + 32 * i) % COLS;
+        const size_t from = (size_t)__shfl_sync(0xffffffffu, row, r) * (COLS * 16) + c * 16;
+        const bool exists = __shfl_sync(0xffffffffu, blk, r) >= 0;   // a row that does not exist is filled with zeros
+        const uint32_t at = cell(0, r, c);
+        cp_async16(st + at, reinterpret_cast<const uint8_t*>(a.k_cache) + from, exists);
+        cp_async16(st + Shape::ROWS_BYTES + at, reinterpret_cast<const uint8_t*>(a.v_cache) + from, exists);
+      }
+      if (KV8 && a.k_scale && lane < 16) cp_async4(scale_ring + to * 32 + lane, a.k_scale + row, blk >= 0);
+      if (KV8 && a.v_scale && lane < 16) cp_async4(scale_ring + to * 32 + 16 + lane, a.v_scale + row, blk >= 0);
+      if (++to == STAGES) to = 0;
+      ahead += SPAN;
+    }
+    cp_async_commit();                                             // one group per call, so that the loop can count them
+  };
   auto request = [&](int place) {
+    if (!WHOLE) return request_rows(place);
     if (ahead >= j_end) return;
     const int blk = checked_page(bt[page_at], a.num_blocks);
     there |= (uint32_t)(blk >= 0) << place;
@@ -713,8 +745,6 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};  // heads 2 t4 and 2 t4 + 1; sums of this lane's tokens
   const float sl2 = a.scale * 1.4426950408889634f;
   constexpr float RAISE = 8.0f;
-  // Address of row r, 16-byte column c of 16 swizzled rows.  ldmatrix: lanes 8 i .. 8 i + 7 give the rows of matrix i.
-  auto cell = [](uint32_t base, int r, int c) { return base + (c >> 3) * 2048 + r * 128 + (((c & 7) ^ (r & 7)) << 4); };
   const int lr = (lane & 7) + (lane & 8), lc = lane >> 4;            // K: matrices = tokens 0-7, 8-15 of a column, then of the next
   const int vr = (lane & 7) + ((lane >> 1) & 8), vcol = (lane >> 3) & 1;  // V: matrices = columns c, c + 1 of tokens 0-7, then 8-15
 
@@ -723,15 +753,21 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
   bool ok = true;
   for (int j = j_begin; j < j_end; j += SPAN) {
     request(STAGES - 1);   // into the stage that the step before this one has left
-    ok = __all_sync(0xffffffffu, mbar_wait(&bars[warp][at], parity, 61));
-    if (!ok) break;
+    if (WHOLE) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[warp][at], parity, 61));
+      if (!ok) break;
+    } else {
+      cp_async_wait<STAGES - 1>();
+      __syncwarp();        // the other lanes' copies too
+    }
     const uint32_t ks_at = smem_u32(ring + at * Shape::STEP_BYTES), vs_at = ks_at + Shape::ROWS_BYTES;
     const float* scales = scale_ring + at * 32;
     if (++at == STAGES) at = 0, parity ^= 1;
-    const bool page_there = there & 1;
+    const uint32_t rows = WHOLE ? there & 1 : (uint32_t)rows_there & 0xffff;
     there >>= 1;
-    if (!page_there) continue;
-    const int left = j_end - j;   // tokens of this step that exist, if fewer than 16
+    rows_there >>= 16;
+    if (rows == 0) continue;
+    const int left = WHOLE ? j_end - j : STEP;   // tokens of this step that exist, if fewer than 16
     // S: tokens g and g + 8 (rows), heads 2 t4 and 2 t4 + 1 (columns)
     float s[2][4];
 #pragma unroll
@@ -761,7 +797,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     for (int h = 0; h < 2; ++h) {
       const float ks = KV8 && a.k_scale ? scales[g + 8 * h] : 1.0f;
       if (KV8 && a.v_scale) vs[h] = scales[16 + g + 8 * h];
-      const bool seen = g + 8 * h < left;
+      const bool seen = WHOLE ? g + 8 * h < left : (rows >> (g + 8 * h)) & 1;
       if (!seen) vs[h] = 0.0f;
       sc[2 * h] = seen ? (s[0][2 * h] + s[1][2 * h]) * (sl2 * ks) : -INFINITY;
       sc[2 * h + 1] = seen ? (s[0][2 * h + 1] + s[1][2 * h + 1]) * (sl2 * ks) : -INFINITY;
@@ -790,6 +826,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     }
     const uint32_t p0 = movmatrix_trans(pack_bf16(p[0], p[1])), p1 = movmatrix_trans(pack_bf16(p[2], p[3]));
     // Rows past the end hold whatever their page holds: a probability of zero does not remove an infinity or NaN, so V is zeroed.
+    // (Rows that the lanes copied are zeroed on their way.)
     uint32_t keep[2] = {~0u, ~0u};
     if (left < STEP) {
 #pragma unroll
@@ -820,6 +857,7 @@ paged_decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     }
     __syncwarp();  // every lane has read the stage before it is asked for again
   }
+  if (!WHOLE) cp_async_wait_all();
   if (!ok) {       // a wait ran out (recorded): copies under way land before shared memory is used again
     for (int i = 0; i < STAGES; ++i)
       if (there >> i & 1) (void)mbar_wait(&bars[warp][(at + i) % STAGES], parity ^ (at + i >= STAGES), 62);
@@ -969,43 +1007,45 @@ int dispatch_flash(const FlashArgs& a, int hd, int max_q_len, int S, cudaStream_
   return -2;
 }
 
-// The tensor-core kernel copies whole 16-token steps of 16-byte vectors.
-bool decode_mma_fits(const DecodeArgs& a, int D) {
-  const unsigned long long addr = reinterpret_cast<unsigned long long>(a.k_cache) | reinterpret_cast<unsigned long long>(a.v_cache) |
-                                  reinterpret_cast<unsigned long long>(a.k_scale) | reinterpret_cast<unsigned long long>(a.v_scale);
-  return a.page % 16 == 0 && (addr & 15) == 0 && (reinterpret_cast<unsigned long long>(a.q) & 3) == 0 && a.num_blocks > 0 &&
-         (long long)a.num_blocks * a.Hkv * a.page < (1ll << 31);
+// Whether TMA can copy a 16-token step as one box, and its scales as one line: the steps of a page are whole and aligned, and the
+// number of rows is known.
+bool decode_steps_whole(const DecodeArgs& a) {
+  const unsigned long long scales = reinterpret_cast<unsigned long long>(a.k_scale) | reinterpret_cast<unsigned long long>(a.v_scale);
+  return a.page % 16 == 0 && (scales & 15) == 0 && a.num_blocks > 0 && (long long)a.num_blocks * a.Hkv * a.page < (1ll << 31);
 }
-template <int D, bool KV8>
+template <int D, bool KV8, bool WHOLE>
 int launch_decode_mma(const DecodeArgs& a, int B, cudaStream_t stream, bool pdl) {
   constexpr int smem = DecodeShape<D, KV8>::SMEM_BYTES;
   static const cudaError_t configured = [] {
-    cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(paged_decode_mma_kernel<D, KV8, WHOLE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   }();
   if (configured != cudaSuccess) return (int)configured;
-  // 8-bit rows are described as half as many 16-bit elements: the copy only moves bytes
-  const unsigned long long rows = (unsigned long long)a.num_blocks * a.Hkv * a.page, cols = KV8 ? D / 2 : D;
-  CUtensorMap tk, tv;
-  int rc = prism_get_tensor_map(a.k_cache, rows, cols, cols, 16, &tk);
-  if (rc == 0) rc = prism_get_tensor_map(a.v_cache, rows, cols, cols, 16, &tv);
-  if (rc) return rc;
+  CUtensorMap tk = {}, tv = {};
+  if (WHOLE) {
+    // 8-bit rows are described as half as many 16-bit elements: the copy only moves bytes
+    const unsigned long long rows = (unsigned long long)a.num_blocks * a.Hkv * a.page, cols = KV8 ? D / 2 : D;
+    int rc = prism_get_tensor_map(a.k_cache, rows, cols, cols, 16, &tk);
+    if (rc == 0) rc = prism_get_tensor_map(a.v_cache, rows, cols, cols, 16, &tv);
+    if (rc) return rc;
+  }
   DecodeArgs c = a;
   c.clustered = a.counters != nullptr && (a.nsplit == 2 || a.nsplit == 4 || a.nsplit == 8 || a.nsplit == 16);
-  return (int)prism_launch_clusters(paged_decode_mma_kernel<D, KV8>, dim3(B, a.Hkv, a.nsplit), dim3(128), smem, stream, pdl,
+  return (int)prism_launch_clusters(paged_decode_mma_kernel<D, KV8, WHOLE>, dim3(B, a.Hkv, a.nsplit), dim3(128), smem, stream, pdl,
                                     c.clustered ? a.nsplit : 1, tk, tv, c);
 }
 
-// use_mma: tensor-core kernel (larger batches); otherwise the SIMT kernel (lowest latency at batch 1)
+// use_mma: tensor-core kernel; otherwise, and for queries that start at an odd element, the SIMT kernel
 template <int D, bool KV8>
 int dispatch_decode(const DecodeArgs& a, int B, cudaStream_t stream, bool pdl, bool use_mma) {
   dim3 grid(B, a.Hkv, a.nsplit), block(128);
-  if (use_mma && decode_mma_fits(a, D)) {
+  if (use_mma && (reinterpret_cast<uintptr_t>(a.q) & 3) == 0) {
     switch (a.Hq / a.Hkv) {
       case 1:
       case 2:
       case 4:
-      case 8: return launch_decode_mma<D, KV8>(a, B, stream, pdl);
+      case 8:
+        return decode_steps_whole(a) ? launch_decode_mma<D, KV8, true>(a, B, stream, pdl) : launch_decode_mma<D, KV8, false>(a, B, stream, pdl);
     }
     return -3;
   }
