@@ -196,17 +196,19 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_kernel(const AddNormArgs a) 
 }
 
 // The form of add+RMSNorm for rows of 16-byte vectors (hidden size a multiple of 8, at most 8192), bf16 delta rows or fp32 slabs.
-// One CTA per row, NV vectors per thread.  Every load of the row is issued before its first store: residual_out may be residual_in,
-// so a load that follows a store in the program also follows it in time, and a loop that reads, adds and writes one vector after the
-// other waits for memory once per vector (1616 x 4096: 39 -> 12 us, 5100 x 4096: 165 -> 55 us; 128 rows of 4 slabs: 9 -> 4 us).
+// One CTA per row, or ROWS rows of one warp each; NV vectors per thread.  Every load of the row is issued before its first store:
+// residual_out may be residual_in, so a load that follows a store in the program also follows it in time, and a loop that reads, adds and
+// writes one vector after the other waits for memory once per vector (1616 x 4096: 39 -> 12 us, 5100 x 4096: 165 -> 55 us).
 // The norm weights come from no kernel and are read before the wait.  Same rounding points as add_rmsnorm_kernel.
+// SLABS: 0 none; 1 added as they come, four loads ahead where four are left; 4 four at a time, absent ones masked.  Which is faster
+// depends on rows and slabs (launch_rows_by_size).
 // ---------------------------------------------------------------------------------
 constexpr int RN_MAX = 8192;
-template <int NV, bool SLABS>
+template <int NV, int SLABS, int ROWS>
 __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNormArgs a) {
   __shared__ float red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int t = blockIdx.x, H = a.H, nvec = H >> 3;
+  const int t = ROWS == 1 ? blockIdx.x : blockIdx.x * ROWS + threadIdx.y, H = a.H, nvec = H >> 3;
   const size_t base = (size_t)t * H;
   pdl_launch_dependents();
   uint4 w[NV], r[NV], e[NV], v[NV];
@@ -218,6 +220,7 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
     }
   }
   pdl_wait();
+  if (ROWS > 1 && t >= a.T) return;
   const int ex = a.extra != nullptr ? a.extra_index[t] : -1;
   float4 lo[NV], hi[NV];
 #pragma unroll
@@ -226,12 +229,13 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
     if (i < nvec) {
       if (a.residual_in != nullptr) r[k] = reinterpret_cast<const uint4*>(a.residual_in + base)[i];
       if (ex >= 0) e[k] = reinterpret_cast<const uint4*>(a.extra + (size_t)ex * H)[i];
-      if (!SLABS) v[k] = reinterpret_cast<const uint4*>(a.x_in + base)[i];
+      if (SLABS == 0) v[k] = reinterpret_cast<const uint4*>(a.x_in + base)[i];
     }
   }
-  if (SLABS) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) lo[k] = hi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = 0; k < NV; ++k) lo[k] = hi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [](float4& sum, const float4& x) { sum.x += x.x, sum.y += x.y, sum.z += x.z, sum.w += x.w; };
+  if (SLABS == 1) {
 #pragma unroll 4
     for (int p = 0; p < a.P; ++p) {
       const float4* src = reinterpret_cast<const float4*>(a.partials + (size_t)p * a.slab_stride + base);
@@ -240,8 +244,28 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
         const int i = threadIdx.x + blockDim.x * k;
         if (i < nvec) {
           const float4 x = __ldcg(src + 2 * i), y = __ldcg(src + 2 * i + 1);
-          lo[k].x += x.x, lo[k].y += x.y, lo[k].z += x.z, lo[k].w += x.w;
-          hi[k].x += y.x, hi[k].y += y.y, hi[k].z += y.z, hi[k].w += y.w;
+          add(lo[k], x), add(hi[k], y);
+        }
+      }
+    }
+  } else if (SLABS > 1) {
+    constexpr int U = SLABS > 1 ? SLABS : 1;
+    for (int p0 = 0; p0 < a.P; p0 += U) {
+      float4 x[U][NV], y[U][NV];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float4* src = reinterpret_cast<const float4*>(a.partials + (size_t)(p0 + u) * a.slab_stride + base);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+          const int i = threadIdx.x + blockDim.x * k;
+          if (p0 + u < a.P && i < nvec) x[u][k] = __ldcg(src + 2 * i), y[u][k] = __ldcg(src + 2 * i + 1);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (p0 + u < a.P) {
+#pragma unroll
+          for (int k = 0; k < NV; ++k) add(lo[k], x[u][k]), add(hi[k], y[u][k]);
         }
       }
     }
@@ -252,7 +276,7 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
     const int i = threadIdx.x + blockDim.x * k;
     if (i < nvec) {
       __nv_bfloat162* vp = reinterpret_cast<__nv_bfloat162*>(&v[k]);
-      if (SLABS) {
+      if (SLABS > 0) {
         vp[0] = __floats2bfloat162_rn(lo[k].x, lo[k].y);
         vp[1] = __floats2bfloat162_rn(lo[k].z, lo[k].w);
         vp[2] = __floats2bfloat162_rn(hi[k].x, hi[k].y);
@@ -281,9 +305,12 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
   }
   if (a.out == nullptr) return;
   ss = warp_sum(ss);
-  if (lane == 0) red[warp] = ss;
-  __syncthreads();
-  const float rstd = rsqrtf(warp_sum(lane < warps ? red[lane] : 0.0f) / (float)H + a.eps);
+  if (ROWS == 1) {
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    ss = warp_sum(lane < warps ? red[lane] : 0.0f);
+  }
+  const float rstd = rsqrtf(ss / (float)H + a.eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int i = threadIdx.x + blockDim.x * k;
@@ -301,11 +328,22 @@ __global__ void __launch_bounds__(1024 / NV) add_rmsnorm_rows_kernel(const AddNo
     }
   }
 }
-template <int NV>
+template <int NV, int SLABS>
 static int launch_add_rmsnorm_rows(const AddNormArgs& a, cudaStream_t stream, bool pdl) {
   const int threads = ((a.H / 8 + NV - 1) / NV + 31) / 32 * 32;
-  return (int)(a.P > 0 ? prism_launch(add_rmsnorm_rows_kernel<NV, true>, dim3(a.T), dim3(threads), 0, stream, pdl, a)
-                       : prism_launch(add_rmsnorm_rows_kernel<NV, false>, dim3(a.T), dim3(threads), 0, stream, pdl, a));
+  if (a.H <= 512 && threads == 32 && a.T > 148)
+    return (int)prism_launch(add_rmsnorm_rows_kernel<NV, SLABS, 4>, dim3((a.T + 3) / 4), dim3(32, 4), 0, stream, pdl, a);
+  return (int)prism_launch(add_rmsnorm_rows_kernel<NV, SLABS, 1>, dim3(a.T), dim3(threads), 0, stream, pdl, a);
+}
+// Up to one row per SM: a vector per thread, the shortest chain.  More rows: few enough threads that several rows share an SM; a warp that
+// has a row of at most 512 to itself shares its CTA with three others (8192 x 128: 9.2 us with one warp, 3.4 with four; 2048 x 512: 2.8
+// and 2.3; 1000 rows of 1024 with a residual: 3.4 and 3.8).
+// Slabs: a vector per thread whatever the number of rows (300 x 1024, 8 slabs: four vectors 15.2 us, one 4.6; 300 x 4096: 16.6 and 11.7).
+// Over at most 148 rows fewer than 8 of them, or wide ones, add fastest as they come (1 x 4096, 2 slabs: 2.2 us, masked 2.5; 32 x 5120, 12
+// slabs: 7.0 and 9.7).
+static int launch_rows_by_size(const AddNormArgs& a, cudaStream_t stream, bool pdl) {
+  if (a.P > 0) return a.T <= 148 && (a.P < 8 || a.H > 4096) ? launch_add_rmsnorm_rows<1, 1>(a, stream, pdl) : launch_add_rmsnorm_rows<1, 4>(a, stream, pdl);
+  return a.T <= 148 || a.H <= 256 ? launch_add_rmsnorm_rows<1, 0>(a, stream, pdl) : launch_add_rmsnorm_rows<4, 0>(a, stream, pdl);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1014,12 +1052,12 @@ static int add_rmsnorm_impl(const void* partials, long long slab_stride, int P, 
     const unsigned long long addr = reinterpret_cast<unsigned long long>(x_in) | reinterpret_cast<unsigned long long>(residual_in) |
                                     reinterpret_cast<unsigned long long>(residual_out) | reinterpret_cast<unsigned long long>(extra) |
                                     reinterpret_cast<unsigned long long>(weight) | reinterpret_cast<unsigned long long>(out);
-    if (n_wait == 0 && !packed && H % 8 == 0 && H <= RN_MAX && (addr & 15ull) == 0 &&
-        (P > 0 ? (slab_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(partials) & 15) == 0) : x_in != nullptr)) {
-      // up to one row per SM: a vector per thread, the shortest chain; more: few enough threads that several rows share an SM
-      if (T <= 148) return launch_add_rmsnorm_rows<1>(a, STREAM(stream), pdl != 0);
-      return launch_add_rmsnorm_rows<4>(a, STREAM(stream), pdl != 0);
-    }
+    // eight slabs or more of few short rows: the wide CTA below, four elements per thread, has twice the loads under way (1 x 4096, 8
+    // slabs: 3.0 us, by vectors 3.4; 64 x 4096: 4.9 and 5.0)
+    const bool wide = P >= 8 && H <= 4096 && (T <= 64 || (long long)T * H <= 1 << 16);
+    if (n_wait == 0 && !packed && !wide && H % 8 == 0 && H <= RN_MAX && (addr & 15ull) == 0 &&
+        (P > 0 ? (slab_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(partials) & 15) == 0) : x_in != nullptr))
+      return launch_rows_by_size(a, STREAM(stream), pdl != 0);
   }
   // few rows: one wide CTA per row so every element has its own thread; many rows: 256 threads
   int threads = T <= 64 ? 1024 : 256;
