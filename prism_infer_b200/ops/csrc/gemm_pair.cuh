@@ -285,8 +285,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             uint32_t ru[16];
             tmem_ld16(t_lane + a.bn / 2 + c0, ru);
             tmem_ld_wait();
+            // Rows past the last token are zeros, for which the unit's division takes its slow path: 257 tokens, 1024 -> 2 x 6144 took 33 us
+            // with them, 512 tokens 22.  One branch for the row: one per element cost full tiles 3 to 10 %.
+            if (row0 + lane < a.T) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = glu(__uint_as_float(r[j]), __uint_as_float(ru[j]), a.act, a.glu_limit);
+              for (int j = 0; j < 16; ++j) v[j] = glu(__uint_as_float(r[j]), __uint_as_float(ru[j]), a.act, a.glu_limit);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = 0.0f;
+            }
           } else {
             const int f = f0 + c0;
             int act = a.act;

@@ -679,3 +679,12 @@ def test_add_rmsnorm_time_of_slabs_and_of_short_rows(cuda_device):
     short, long = (replay_us([lambda: ops.rmsnorm(x, w[:x.shape[1]], 1e-6)] * 8)
                    for x in (torch.zeros(8192, n, dtype=torch.bfloat16, device="cuda") for n in (128, 1024)))
     assert short < 0.6 * long, (short, long)
+
+
+def test_gated_time_of_a_ragged_token_tile(cuda_device):
+    """257 tokens run in the two token tiles of 512: the rows past the last token cost nothing in the epilogue (1.5 times the full tiles'
+    time while they took part)."""
+    ws = rand_bf16(2 * 6144 * 8, 1024, scale=1 / 32, seed=111).cuda().view(8, 2 * 6144, 1024)
+    x = rand_bf16(512, 1024, seed=112).cuda()
+    ragged, full = (replay_us([lambda i=i: ops.gate_up_swiglu(x[:n], ws[i]) for i in range(8)]) for n in (257, 512))
+    assert ragged < 1.2 * full, (ragged, full)
