@@ -982,11 +982,6 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
       a.peer_flag[p] = push->peer_flag[p];
     }
   }
-  CUtensorMap tw, tx;
-  int rc = get_tensor_map(W, (unsigned long long)w_rows_total, (unsigned long long)K, (unsigned long long)ldw, BM, &tw);
-  if (rc) return rc;
-  rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, (unsigned)bn, &tx);
-  if (rc) return rc;
   const int m_tiles = (M + BM - 1) / BM;
   const bool p = pdl != 0;
   const bool plan_own = push == nullptr && bn_override <= 0 && stages_override <= 0 && g_persistent_min_tokens > 0;
@@ -1016,6 +1011,9 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
     g.sec = a.sec;
     return launch_pair(W, X, K, ldw, ldx, w_rows_total, g, stream, p);
   }
+  CUtensorMap tw, tx;
+  int rc = get_tensor_map(W, (unsigned long long)w_rows_total, (unsigned long long)K, (unsigned long long)ldw, BM, &tw);
+  if (rc) return rc;
   if (plan_own && T >= g_persistent_min_tokens && splits == 1 && !out_f32 && sections == nullptr) {
     PersistArgs pa;
     pa.groups = nullptr;
@@ -1048,11 +1046,12 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
     // dual: two accumulators per tile, so 128 tokens per tile keep two tiles in TMEM
     const int pbn = dual ? 128 : 256;
     pa.n_tiles = (T + pbn - 1) / pbn;
-    CUtensorMap txp;
-    rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, (unsigned)pbn, &txp);
+    rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, (unsigned)pbn, &tx);
     if (rc) return rc;
-    return dual ? launch_persistent<128, true>(tw, txp, pa, stream, p) : launch_persistent<256, false>(tw, txp, pa, stream, p);
+    return dual ? launch_persistent<128, true>(tw, tx, pa, stream, p) : launch_persistent<256, false>(tw, tx, pa, stream, p);
   }
+  rc = get_tensor_map(X, (unsigned long long)T, (unsigned long long)K, (unsigned long long)ldx, (unsigned)bn, &tx);
+  if (rc) return rc;
 #define PRISM_GEMM_CASE(BN_)                                                                            \
   case BN_:                                                                                             \
     return dual ? launch_gemm<BN_, true>(tw, tx, a, m_tiles, splits, stages_override, stream, p)       \
@@ -1296,6 +1295,12 @@ PRISM_API int prism_gemm_effective_splits(int K, int splits) {
   if (splits > kb_total) splits = kb_total;
   const int per = (kb_total + splits - 1) / splits;
   return (kb_total + per - 1) / per;
+}
+
+// How many tensor maps are kept.
+PRISM_API int prism_gemm_tensor_maps() {
+  std::lock_guard<std::mutex> lock(g_map_mutex);
+  return (int)g_maps.size();
 }
 
 PRISM_API void prism_gemm_clear_tensor_maps() {

@@ -64,6 +64,7 @@ _SIGNATURES = {
     "prism_flash_attention_tc_kv": "plpplplppp" "liiiiiiifpi",
     "prism_gemm_effective_splits": "ii",
     "prism_gemm_clear_tensor_maps": "",
+    "prism_gemm_tensor_maps": "",
     "prism_add_rmsnorm": "plipppppppiifpi",
     "prism_layernorm": "ppppiifpi",
     "prism_qk_norm_rope_store": "pplilpppppplpppppiiiiiiiifipi",

@@ -688,3 +688,14 @@ def test_gated_time_of_a_ragged_token_tile(cuda_device):
     x = rand_bf16(512, 1024, seed=112).cuda()
     ragged, full = (replay_us([lambda i=i: ops.gate_up_swiglu(x[:n], ws[i]) for i in range(8)]) for n in (257, 512))
     assert ragged < 1.2 * full, (ragged, full)
+
+
+@pytest.mark.parametrize("T,M", [(300, 512), (5, 512), (700, 1000)])
+def test_gemm_asks_for_the_maps_of_the_kernel_that_runs(cuda_device, T, M):
+    """Two tensor maps a product, one of them for new activations only."""
+    x, w = rand_bf16(T, 256, seed=121).cuda(), rand_bf16(M, 256, seed=122).cuda()
+    native.lib().prism_gemm_clear_tensor_maps()
+    ops.linear(x, w)
+    assert native.lib().prism_gemm_tensor_maps() == 2
+    ops.linear(x.clone(), w)
+    assert native.lib().prism_gemm_tensor_maps() == 3
