@@ -53,32 +53,30 @@ def _pdl() -> int:
 
 
 # ------------------------------------------------------------------------------- GEMM
-SPLIT_K_MAX_TOKENS = 511  # from 512 tokens the persistent GEMM (several tiles per CTA) takes over
+SPLIT_K_MAX_TOKENS = 511  # longer prompts have tiles for every SM without splitting K
 
 
 def choose_splits(m: int, k: int, tokens: int) -> int:
     """Split-K factor that fills the 148 SMs: for a weight-streaming GEMM (at most 128 tokens, one token
-    tile) and for the short prefills above it (up to 511 tokens, one or two token tiles), where a
+    tile) and for the short prefills above it (up to 511 tokens, two to four tiles of 128 tokens), where a
     row-parallel projection with 32 weight tiles would otherwise keep a fifth of the SMs busy."""
     if tokens > SPLIT_K_MAX_TOKENS:
         return 1
-    tiles = (m + 127) // 128
-    if tokens > 128:
-        tiles *= (tokens + 255) // 256
+    tiles = (m + 127) // 128 * (1 if tokens <= 128 else (tokens + 127) // 128)
     kb = (k + 63) // 64
     # one CTA per SM is resident (the operand ring fills shared memory), so more CTAs than
     # SMs means a second, mostly empty wave: stay at or below the SM count
     want = max(1, SM_COUNT // tiles)
-    if tokens > 128 and tiles >= 16:
-        # the SM pairs' kernel picks its tile width too: two slabs of a 4096-wide projection fill the pairs with 128 columns, and
-        # further slabs cost more in 32-bit partials than their shorter sums give
-        want = min(want, 2)
+    if tokens > 128:
+        # Where 256-token tiles leave half the SMs idle the sum stays in two 32-bit slabs.  With the norm that adds them, 230 tokens:
+        # 2048 -> 2048 four slabs 13.3 us (two on SM pairs 12.7), 6144 -> 2048 17.3 (18.5); 384 tokens 13.8 (15.4) and 18.5 (21.7)
+        want = max(want, min(2, SM_COUNT // ((m + 127) // 128 * ((tokens + 255) // 256))))
     return max(1, min(want, kb // 4 if kb >= 8 else 1, 16))
 
 
 def narrow_splits(m: int, k: int, tokens: int) -> int:
     """Split-K factor of a long prompt's projection to few features (a router, a side gate), whose output tiles would keep
-    only some of the SMs busy: 2048 tokens, 4096 -> 256 took 32 us on 16 SMs.  1: run it as rows."""
+    only some of the SMs busy (2048 tokens, 4096 -> 256: 8 tiles of a pair of SMs).  1: run it as rows."""
     tiles = -(-m // 128) * -(-tokens // 256)
     return max(1, min(SM_COUNT // tiles, -(-k // 64) // 8, 8)) if tokens > SPLIT_K_MAX_TOKENS else 1
 

@@ -833,19 +833,38 @@ int launch_persistent(const CUtensorMap& tw, const CUtensorMap& tx, PersistArgs&
   return (int)prism_launch(gemm_wx_persistent_kernel<BN, DUAL, ROWMAJOR, GROUPED>, dim3(grid), dim3(GEMM_THREADS), smem, stream, pdl, tw, tx, a);
 }
 
+// Rounds that `tiles` take on `places`.
+int rounds_of(long long tiles, int places) { return (int)((tiles + places - 1) / places); }
+
 // Columns of a pair's tile.  A k-block of a tile takes 390 cycles (issue and barriers) or 2.7 per column, whichever is longer
 // (measured over 64 to 256 columns), and the launch as many rounds of tiles as the pairs need: 1616 x 4096 -> 4096 took 44 us with
 // 224 columns (two rounds of a few more columns than half of 256), 47 with 256, 56 with 128.
-int pair_columns(int m_tiles, int columns, bool dual) {
+int pair_columns(int m_tiles, int columns, bool dual, int* best_rounds = nullptr) {
   const int pairs = sm_count() / 2, step = dual ? 64 : 32;
   int best = 64;
   long long best_cost = 0;
   for (int bn = 64; bn <= 256; bn += step) {
-    const long long rounds = ((long long)m_tiles * ((columns + bn - 1) / bn) + pairs - 1) / pairs;
-    const long long cost = rounds * ((bn < 144 ? 144 : bn) + 8);
-    if (best_cost == 0 || cost < best_cost) best = bn, best_cost = cost;
+    const int rounds = rounds_of((long long)m_tiles * ((columns + bn - 1) / bn), pairs);
+    const long long cost = (long long)rounds * ((bn < 144 ? 144 : bn) + 8);
+    if (best_cost == 0 || cost < best_cost) {
+      best = bn, best_cost = cost;
+      if (best_rounds != nullptr) *best_rounds = rounds;
+    }
   }
   return best;
+}
+
+// Token tile with which fp32 slabs of more than 128 tokens run on single SMs; 0: on SM pairs.  A pair's epilogue stores 32-bit results by
+// lane and the pairs' 256-token tiles waste rows, so single SMs win where their tiles are one round: with 128 tokens always but for the
+// narrowest sums (4096 -> 1152, 257 tokens, 5 slabs: pairs 15.1 us, single SMs 8.8; 1152 -> 256, 129 tokens, 4 slabs: 5.5 and 6.3), with
+// 256 tokens where the pairs need two rounds (4096 -> 1152, 512 tokens, 8 slabs: 17.1 and 13.5).
+int slab_token_tile(int M, int T, int splits) {
+  const int m_tiles = (M + BM - 1) / BM, t_tiles = (T + 255) / 256;
+  int rounds = 1;
+  const int columns = pair_columns(t_tiles * splits, M, false, &rounds);
+  if (M <= 128 || ((T <= 256 || M <= 512) && columns == 64)) return 0;
+  if ((long long)m_tiles * ((T + 127) / 128) * splits <= sm_count()) return 128;
+  return rounds > 1 && (long long)m_tiles * t_tiles * splits <= sm_count() ? 256 : 0;
 }
 
 int launch_pair(const void* W, const void* X, int K, long long ldw, long long ldx, int w_rows, PairArgs& a, cudaStream_t stream, bool pdl) {
@@ -989,7 +1008,10 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
                                       reinterpret_cast<unsigned long long>(residual);
   // SM pairs, tokens on the TMEM lanes: from 129 tokens, where two CTAs have rows of their own, if the epilogue can move 16-byte
   // vectors.  4096 -> 4096: 230 tokens 17 us (split-K form below 33), 1616 tokens 44 us (one-SM persistent form 64).
-  if (plan_own && T > 128 && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 && split_stride % 4 == 0 && (residual == nullptr || ldr % 8 == 0) &&
+  const bool slabs = out_f32 && sections == nullptr && plan_own && T > 128;
+  const int slab_tile = slabs ? slab_token_tile(M, T, splits) : 0;
+  if (slab_tile > 0) bn = slab_tile;
+  if (plan_own && slab_tile == 0 && T > 128 && g_persistent_rowmajor && M % 16 == 0 && ldo % 8 == 0 && split_stride % 4 == 0 && (residual == nullptr || ldr % 8 == 0) &&
       (vec_addr & 15ull) == 0 && (!dual || (bias == nullptr && residual == nullptr)) && (!out_f32 || sections != nullptr || (bias == nullptr && residual == nullptr && act == 0)) &&
       (sections == nullptr || sections_rowmajor)) {
     PairArgs g = {};

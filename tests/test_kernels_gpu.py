@@ -699,3 +699,24 @@ def test_gemm_asks_for_the_maps_of_the_kernel_that_runs(cuda_device, T, M):
     assert native.lib().prism_gemm_tensor_maps() == 2
     ops.linear(x.clone(), w)
     assert native.lib().prism_gemm_tensor_maps() == 3
+
+
+@pytest.mark.parametrize("T,M,K,splits", [(129, 256, 1152, 4), (257, 1152, 4096, 5), (130, 640, 1096, 9), (512, 1152, 4096, 8), (1030, 1160, 2056, 3),
+                                          (385, 1000, 1160, 4), (2050, 136, 72, 1), (511, 4096, 264, 2)])
+def test_slabs_of_prompts_on_either_kernel(cuda_device, T, M, K, splits):
+    """128- and 256-token tiles of single SMs and the SM pairs, ragged tiles, slabs with a shorter last share of K.  A slab's sum is a chain of
+    K / 16 additions, each off by 2^-23 of a running sum that stays below 4."""
+    x, w = rand_bf16(T, K, seed=131), rand_bf16(M, K, scale=K ** -0.5, seed=132)
+    got = ops.linear_partial(x.cuda(), w.cuda(), splits)
+    assert got.shape[0] == ops.effective_splits(K, splits)
+    err = (got.double().sum(0).cpu() - x.double() @ w.double().t()).abs()
+    assert err.max() < 4.0 * (K / 16 + 16) * 2.0 ** -23, err.max()
+
+
+@pytest.mark.parametrize("T,splits,bn", [(257, 5, 128), (512, 8, 256)])
+def test_slabs_of_prompts_take_the_faster_kernel(cuda_device, T, splits, bn):
+    """4096 -> 1152: single SMs where their tiles are one round (the pairs took 1.7 and 1.27 times as long)."""
+    ws = rand_bf16(16 * 1152, 4096, scale=1 / 64, seed=133).cuda().view(16, 1152, 4096)
+    x = rand_bf16(T, 4096, seed=134).cuda()
+    chosen, single = (replay_us([lambda i=i: ops.linear_partial(x, ws[i], splits, bn=n) for i in range(16)]) for n in (0, bn))
+    assert chosen < 1.12 * single, (chosen, single)

@@ -366,3 +366,17 @@ def test_decoder_composed_of_the_layer_modules_matches_the_oracle():
     got = torch.cat((first, second, last))
     assert got.shape == want.shape
     assert float((got - want).abs().max()) < 2e-4, float((got - want).abs().max())
+
+
+def test_split_factors_of_short_prompts_fill_the_sms():
+    """Slabs times 128-token tiles fill the SMs once; two slabs stay where 256-token tiles leave half of them idle.  A number of features that
+    is no multiple of 16 counts like any other (1000 features of 511 tokens had two slabs for 32 tiles)."""
+    for m in (64, 256, 576, 1000, 1152, 2048, 2056, 4096, 5120, 6144, 12288):
+        for tokens in (1, 64, 128, 129, 256, 257, 384, 385, 511):
+            s = ops.choose_splits(m, 8192, tokens)
+            rows, wide = -(-m // 128), 128 if tokens <= 128 else 256
+            tiles, coarse = rows * -(-tokens // 128), rows * -(-tokens // wide)
+            assert s * tiles <= ops.SM_COUNT or s * coarse <= ops.SM_COUNT and s <= 2 or s == 1, (m, tokens, s)
+            assert s == 16 or (s + 1) * tiles > ops.SM_COUNT, (m, tokens, s)
+            assert s > 1 or 2 * coarse > ops.SM_COUNT, (m, tokens, s)
+    assert ops.choose_splits(1000, 4096, 511) == 4 and ops.choose_splits(4096, 4096, 512) == 1
