@@ -720,3 +720,53 @@ def test_slabs_of_prompts_take_the_faster_kernel(cuda_device, T, splits, bn):
     x = rand_bf16(T, 4096, seed=134).cuda()
     chosen, single = (replay_us([lambda i=i: ops.linear_partial(x, ws[i], splits, bn=n) for i in range(16)]) for n in (0, bn))
     assert chosen < 1.12 * single, (chosen, single)
+
+
+@pytest.mark.parametrize("T,M,K", [(4100, 8208, 136), (2300, 16400, 72)])
+def test_gemm_on_sm_pairs_over_many_rounds(cuda_device, T, M, K):
+    """More tiles than four times the pairs: both accumulators are handed back several times and the ring goes round across tiles."""
+    x, w = rand_bf16(T, K, seed=141).cuda(), rand_bf16(M, K, scale=K ** -0.5, seed=142).cuda()
+    close(ops.linear(x, w), x.float() @ w.float().t(), 2e-2, 2e-2, "plain")
+    I = M // 2
+    y = x.double() @ w.double().t()
+    close(ops.gate_up_glu(x, w, "silu"), torch.nn.functional.silu(y[:, :I]) * y[:, I:], 2e-2, 2e-2, "gated")
+
+
+@pytest.mark.parametrize("T,M,K", [(512, 1000, 1160), (1500, 2056, 264), (5000, 520, 72)])
+@pytest.mark.parametrize("form", ["plain", "bias gelu residual", "gated"])
+def test_gemm_of_long_prompts_with_features_on_the_lanes(cuda_device, T, M, K, form):
+    """Feature counts that are no multiple of 16 run on single SMs from 512 tokens, several tiles per CTA."""
+    x, w = rand_bf16(T, K, seed=151), rand_bf16(2 * M if form == "gated" else M, K, scale=K ** -0.5, seed=152)
+    y = x.double() @ w.double().t()
+    if form == "gated":
+        got, want = ops.gate_up_glu(x.cuda(), w.cuda(), "gelu_tanh"), torch.nn.functional.gelu(y[:, :M], approximate="tanh") * y[:, M:]
+    elif form == "plain":
+        got, want = ops.linear(x.cuda(), w.cuda()), y
+    else:
+        b, r = rand_bf16(M, seed=153), rand_bf16(T, M, seed=154)
+        got = ops.linear(x.cuda(), w.cuda(), bias=b.cuda(), act="gelu", residual=r.cuda())
+        want = torch.nn.functional.gelu(y + b.double()) + r.double()
+    close(got, want, 2e-2, 2e-2, form)
+
+
+@pytest.mark.parametrize("T", [150, 700])
+def test_gemm_on_sm_pairs_with_strided_rows(cuda_device, T):
+    """Activations, weights, residual and results that are windows of wider matrices; the columns beside the results stay."""
+    K, M = 264, 528
+    xs, ws, rs = rand_bf16(T, 2 * K, seed=161).cuda(), rand_bf16(M, 3 * K, scale=K ** -0.5, seed=162).cuda(), rand_bf16(T, 2 * M, seed=163).cuda()
+    x, w, r = xs[:, K:], ws[:, K:2 * K], rs[:, M:]
+    out = torch.full((T, 3 * M), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.linear(x, w, residual=r, out=out[:, M:2 * M])
+    close(out[:, M:2 * M], x.float() @ w.float().t() + r.float(), 3e-2, 2e-2, "window")
+    assert bool((out[:, :M] == 7.0).all()) and bool((out[:, 2 * M:] == 7.0).all())
+
+
+@pytest.mark.parametrize("heads,hd", [(16, 72), (3, 68), (24, 128), (5, 36), (1, 4), (2, 256)])
+def test_vit_rope_of_every_head_size(cuda_device, heads, hd):
+    """Heads of 8-byte and of 4-byte accesses, more rows than a block turns at once, fewer than it has threads."""
+    qkv = rand_bf16(37, 3 * heads * hd, seed=171)
+    coords = torch.randint(0, 40, (37, 2), generator=torch.Generator().manual_seed(172)).int()
+    inv = 1.0 / (10000.0 ** (torch.arange(0, hd // 2, 2).float() / (hd // 2)))
+    got = ops.vit_rope(qkv.clone().cuda(), coords.cuda(), inv.cuda(), heads, hd)
+    close(got, ops.vit_rope(qkv.float().clone(), coords, inv, heads, hd), 3e-2, 1e-2, "rotary")
+    assert torch.equal(got.cpu().view(37, 3, -1)[:, 2], qkv.view(37, 3, -1)[:, 2])
