@@ -29,7 +29,8 @@ _PDL = False
 
 
 def set_pdl(enabled: bool) -> None:
-    """Launch kernels with programmatic stream serialization (overlapped prologues)."""
+    """Launch kernels with programmatic stream serialization (overlapped prologues): weights of products and norms are read while the
+    kernel before is still at work, so none of them may be that kernel's output."""
     global _PDL
     _PDL = bool(enabled)
 
@@ -68,8 +69,8 @@ def choose_splits(m: int, k: int, tokens: int) -> int:
     # SMs means a second, mostly empty wave: stay at or below the SM count
     want = max(1, SM_COUNT // tiles)
     if tokens > 128:
-        # Where 256-token tiles leave half the SMs idle the sum stays in two 32-bit slabs.  With the norm that adds them, 230 tokens:
-        # 2048 -> 2048 four slabs 13.3 us (two on SM pairs 12.7), 6144 -> 2048 17.3 (18.5); 384 tokens 13.8 (15.4) and 18.5 (21.7)
+        # Where 256-token tiles leave half the SMs idle the sum stays in two 32-bit slabs.  With the norm that adds them, against two slabs
+        # on SM pairs: 230 tokens, 2048 -> 2048 12.7 -> 11.7 us, 6144 -> 2048 18.7 -> 16.0; 384 tokens 15.5 -> 12.3 and 21.8 -> 17.1
         want = max(want, min(2, SM_COUNT // ((m + 127) // 128 * ((tokens + 255) // 256))))
     return max(1, min(want, kb // 4 if kb >= 8 else 1, 16))
 
@@ -234,7 +235,8 @@ PAGED_PREFILL_TC_ENABLED = True
 # page-reading kernel runs instead (a prefill step over very many long histories), so the scratch stays inside the
 # memory the KV sizing leaves free
 PAGED_PREFILL_TC_MAX_SCRATCH_BYTES = 2 << 30
-# prefill GEMMs of at least this many tokens run the persistent form, tokens on the TMEM lanes
+# prompt GEMMs (more than 128 tokens) run on SM pairs, tokens on the TMEM lanes; what these do not take (rows that are not whole 16-byte
+# vectors) runs the single-SM persistent form from this many tokens.  0 tokens: neither of them
 PERSISTENT_ROWMAJOR = True
 PERSISTENT_MIN_TOKENS = 512
 # shared-memory cap of decode-sized GEMM launches (0 = none)
@@ -583,7 +585,11 @@ def embed(ids: torch.Tensor, table: torch.Tensor, *, visual: Optional[torch.Tens
 def decode_splits(batch: int, num_kv_heads: int) -> int:
     """Blocks that share the cached tokens of one (sequence, KV head): a power of two, whose blocks form a cluster and merge in
     shared memory, at most 16 (the largest cluster) and at most 256 blocks in all (two and three of them fit an SM, and a call of more
-    than one round is slower: 8 sequences of up to 3000 tokens, 8 KV heads: 20 us with 2, 18 with 4, 22 with 8, 43 with 16)."""
+    than one round is slower: 8 sequences of up to 3000 tokens, 8 KV heads: 20 us with 2, 18 with 4, 22 with 8, 43 with 16).
+
+    32 splits, merged through memory, lose up to 16 K tokens and win where 16 blocks stream for long: one sequence, 8 KV heads, bf16:
+    4096 tokens 8.5 us with 16, 13.7 with 32; 131072 tokens 86 and 91, in 8 bits 133 and 85; one KV head 69 and 47, in 8 bits 99 and 62.
+    The length is not known here, and at 16 every length is 1.3 to 2.6 times as fast as with the kernel before (16 K to 128 K tokens)."""
     n = 1
     while n < 16 and 2 * n * batch * num_kv_heads <= 256:
         n *= 2

@@ -7,15 +7,16 @@
 //
 // The issuing threads were the other half of it.  Behind lane == 0 an MMA took 90 cycles to issue, and a 64-bit division for the ring
 // stage 400: 64-column tiles cost as much as 256-column ones.  With elect.sync and a carried stage a k-block is bound by its 512
-// tensor cycles (256 columns).  Measured, start -> now (single-SM form with feature or token rows before): 2048 x 4096 -> 2 x 12288
-// gated 344 -> 266 us (1548 TFLOP/s, the power limit's rate), 7500 tokens 1296 -> 952; 1616 x 12288 -> 4096 177 -> 133; 6272 x 1152
-// -> 4304 with GELU 60 -> 57; 230 x 4096 -> 6144 33 -> 19.
+// tensor cycles (256 columns).  Measured, single-SM kernels that issue behind lane == 0 -> this kernel (graph replays, weights from
+// memory): 2048 x 4096 -> 2 x 12288 gated 348 -> 270 us (1528 TFLOP/s, the power limit's rate), 7500 tokens 1263 -> 987; 1616 x 12288 ->
+// 4096 174 -> 126; 230 x 4096 -> 6144 33 -> 19.
 //
 // Tokens lie on the TMEM lanes, so a thread of the epilogue gets 16 features of one token row at a time.  Eight epilogue warps (two
 // per lane quarter) drain one accumulator while the next tile fills the other.  bf16 results turn in shared memory (32 rows x 64
 // features a warp, columns XORed with the row against bank conflicts) and leave, with the residual, as whole 128-byte lines: lanes
 // that store 16 bytes each into 32 rows cost 32 requests to L2 per instruction, and short products were bound by them (6272 x 1152 -> 3456
-// with bias: 61 -> 51 us; 1152 -> 1152 with bias and residual: 35 -> 26).
+// with bias: 61 us by lane, 51 turned, in one run; in the run of the figures above 66 on single SMs and 44 here, 1152 -> 1152 with
+// residual 42 and 29).
 //
 // The TMA loads carry cta_group::2 only so that both CTAs' copies may report to the even CTA's barrier; every copy goes to its own CTA.
 // MMA completion is reported to the even CTA, whose producer and epilogue pass it on to the odd one.

@@ -800,8 +800,8 @@ int launch_gemm(const CUtensorMap& tw, const CUtensorMap& tx, GemmArgs& a, int m
 }
 
 
-int g_persistent_min_tokens = 512;  // 0 disables the persistent form
-int g_persistent_rowmajor = 1;      // 1: tokens on the TMEM lanes for the non-dual persistent GEMM
+int g_persistent_min_tokens = 512;  // fewest tokens of the single-SM persistent form; 0: neither it nor the SM pairs
+int g_persistent_rowmajor = 1;      // 0: no SM pairs, whose tokens lie on the TMEM lanes
 int g_sm_count = 0;
 
 int sm_count() {
@@ -961,7 +961,7 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
   a.out_f32 = out_f32;
   a.act = act;
   a.sec.n = 0;
-  bool sections_rowmajor = true;  // the persistent row-major epilogue can serve them
+  bool sections_rowmajor = true;  // the SM pairs' epilogue can serve them
   if (sections != nullptr) {
     if (dual || splits > 1 || push != nullptr || residual != nullptr || act != 0) return -8;
     a.sec = *sections;
@@ -1007,7 +1007,8 @@ static int gemm_wx_impl(const void* W, const void* X, void* out, int M, int T, i
   const unsigned long long vec_addr = reinterpret_cast<unsigned long long>(out) | reinterpret_cast<unsigned long long>(bias) |
                                       reinterpret_cast<unsigned long long>(residual);
   // SM pairs, tokens on the TMEM lanes: from 129 tokens, where two CTAs have rows of their own, if the epilogue can move 16-byte
-  // vectors.  4096 -> 4096: 230 tokens 17 us (split-K form below 33), 1616 tokens 44 us (one-SM persistent form 64).
+  // vectors.  4096 -> 4096 in bf16: 230 tokens 18 us (one tile per SM 32), 1616 tokens 44 us (one-SM persistent form 62).  Slabs: by the
+  // rule of slab_token_tile.
   const bool slabs = out_f32 && sections == nullptr && plan_own && T > 128;
   const int slab_tile = slabs ? slab_token_tile(M, T, splits) : 0;
   if (slab_tile > 0) bn = slab_tile;
@@ -1298,7 +1299,7 @@ PRISM_API int prism_gemm_set_persistent_rowmajor(int on) {
   return 0;
 }
 
-// Smallest token count that uses the persistent kernel (0 = never).
+// Fewest tokens of the single-SM persistent kernel (0: neither it nor the SM pairs).
 PRISM_API int prism_gemm_set_persistent_min_tokens(int tokens) {
   g_persistent_min_tokens = tokens;
   return 0;

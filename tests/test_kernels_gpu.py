@@ -440,12 +440,12 @@ def test_vision_pointwise(cuda_device):
 
 @pytest.mark.parametrize("T,M,K", [(3000, 2000, 320), (6272, 1152, 1152), (777, 4304, 1152)])
 def test_gemm_persistent_matches_tiled_kernel(cuda_device, T, M, K):
-    """The persistent form (several tiles per CTA, two TMEM accumulators) gives the same bits as
-    the one-tile-per-CTA kernel for every epilogue, and both match the fp32 reference."""
+    """The persistent form (on SM pairs: several tiles per pair, two TMEM accumulators) gives the same
+    bits as the one-tile-per-CTA kernel for every epilogue, and both match the fp32 reference."""
     x, w = rand_bf16(T, K, seed=21).cuda(), rand_bf16(M, K, scale=K ** -0.5, seed=22).cuda()
     b, r = rand_bf16(M, seed=23).cuda(), rand_bf16(T, M, seed=24).cuda()
     for kw in (dict(), dict(bias=b, act="gelu_tanh"), dict(bias=b, residual=r)):
-        got = ops.linear(x, w, **kw)            # T >= 512: persistent kernel
+        got = ops.linear(x, w, **kw)            # the SM pairs
         want = ops.linear(x, w, bn=256, **kw)   # explicit tile size: one tile per CTA
         torch.cuda.synchronize()
         assert torch.equal(got, want), f"persistent vs tiled differ for {list(kw)}"
