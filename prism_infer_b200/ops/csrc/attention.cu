@@ -1069,6 +1069,7 @@ PRISM_API int prism_paged_decode(const void* q, const void* k_cache, const void*
                                  void* stream, int pdl) {
   if (B <= 0) return 0;
   if (Hq <= 0 || Hkv <= 0 || Hq % Hkv || page <= 0 || max_blocks <= 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) return -4;  // rows are read as 16-byte vectors
   DecodeArgs a;
   a.q = (const bf16*)q;
   a.k_cache = k_cache;

@@ -770,3 +770,14 @@ def test_vit_rope_of_every_head_size(cuda_device, heads, hd):
     got = ops.vit_rope(qkv.clone().cuda(), coords.cuda(), inv.cuda(), heads, hd)
     close(got, ops.vit_rope(qkv.float().clone(), coords, inv, heads, hd), 3e-2, 1e-2, "rotary")
     assert torch.equal(got.cpu().view(37, 3, -1)[:, 2], qkv.view(37, 3, -1)[:, 2])
+
+
+def test_paged_decode_refuses_a_cache_that_is_not_whole_vectors(cuda_device):
+    """Rows are read as 16-byte vectors: a cache that starts between two of them is refused before anything is launched."""
+    table, ctx = torch.zeros(1, 1, dtype=torch.int32, device="cuda"), torch.ones(1, dtype=torch.int32, device="cuda")
+    q = torch.zeros(1, 4, 128, dtype=torch.bfloat16, device="cuda")
+    for page in (16, 24):
+        cache = torch.zeros(2 * page * 128 + 8, dtype=torch.bfloat16, device="cuda")
+        with pytest.raises(native.NativeError):
+            native.call("prism_paged_decode", q.data_ptr(), cache.data_ptr() + 8, cache.data_ptr(), None, None, table.data_ptr(), ctx.data_ptr(),
+                        None, None, q.data_ptr(), None, 1, 4, 1, 128, page, 1, 1, 1, ops.KV_BF16, 0.1, 1, ops._s(), 0)
