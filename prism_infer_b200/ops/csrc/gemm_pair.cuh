@@ -286,15 +286,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             uint32_t ru[16];
             tmem_ld16(t_lane + a.bn / 2 + c0, ru);
             tmem_ld_wait();
-            // Rows past the last token are zeros, for which the unit's division takes its slow path: 257 tokens, 1024 -> 2 x 6144 took 33 us
-            // with them, 512 tokens 22.  One branch for the row: one per element cost full tiles 3 to 10 %.
-            if (row0 + lane < a.T) {
+            // Rows past the last token are zeros, for which the unit's division takes its slow path (257 tokens, 1024 -> 2 x 6144: 33 us,
+            // 512 tokens 22): they get another gate.  A branch around the row made the plain products' epilogue slower (6272 x 1152 -> 4304
+            // with GELU 57.1 -> 58.1), one around each element full gated tiles (3 to 10 %).
+            const bool live = row0 + lane < a.T;
 #pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = glu(__uint_as_float(r[j]), __uint_as_float(ru[j]), a.act, a.glu_limit);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-            }
+            for (int j = 0; j < 16; ++j) v[j] = glu(live ? __uint_as_float(r[j]) : 1.0f, __uint_as_float(ru[j]), a.act, a.glu_limit);
           } else {
             const int f = f0 + c0;
             int act = a.act;
